@@ -459,31 +459,31 @@ int lfx_batch_set_wait_limit(lfx_batch* b, double seconds);
 /* ------------------------------------------------------------------ many right-hand sides
  * One operator applied to, and solved for, nrhs right-hand sides at once (no
  * counterpart in the reference, whose solvers take one field_vector_type).
- * The per-cell product becomes an (nrhs x 8) by (8 x 8) small GEMM on the
- * tensor cores, in TF32 or BF16 with FP32 accumulation. Operators with the
+ * The local matrices are summed once into column stencils (27 coefficients a
+ * row on a quadrilateral mesh), which are applied in FP32. Operators with the
  * lowest-order nodal (W0) dofmap only: ndf = 8, map_to == map_from, dofs 4..7
  * one level above dofs 0..3. */
 typedef struct lfx_mrhs lfx_mrhs;
 enum { LFX_MRHS_TF32 = 1, LFX_MRHS_BF16 = 2 };
-/* From an FP64 (or FP32) LMA operator: its matrices rounded to `kind`, the
- * cell columns split into patches of about cells_per_patch (0: 16). nrhs is
- * 16, 32 or 64. */
+/* From an FP64 (or FP32) LMA operator. kind is the least precision the caller
+ * takes for the products (both kinds compute in FP32); the cell columns are
+ * split into patches of about cells_per_patch (0: 16). nrhs is 16, 32 or 64. */
 int lfx_mrhs_create(const lfx_op* op, int32_t kind, int32_t nrhs, int32_t cells_per_patch,
                     lfx_mrhs** out);
 int lfx_mrhs_destroy(lfx_mrhs* m);
-/* patches, cell levels computed per apply (halo cells of two patches count
- * twice), most vertex columns one patch owns, most colours in one patch, and
- * the bytes of the rounded matrices */
+/* patches, cell levels that touch the vertex columns of each patch (halo cells
+ * of two patches count twice), most vertex columns one patch owns, most
+ * colours in one patch, and the bytes of the stencils */
 int lfx_mrhs_info(const lfx_mrhs* m, int32_t* npatch, int64_t* cell_levels, int32_t* max_owned,
                   int32_t* max_colours, int64_t* matrix_bytes);
 /* y = A x for device arrays x, y of undf x nrhs FP32 values, dof-major
- * (element (dof, rhs) at dof * nrhs + rhs); x and y must differ */
+ * (element (dof, rhs) at dof * nrhs + rhs), 16-byte aligned (x: 8 bytes for 16
+ * right-hand sides); x and y must differ */
 int lfx_mrhs_apply(lfx_mrhs* m, const float* x, float* y);
 /* mean time of one apply over reps applies (after one untimed), microseconds */
 int lfx_mrhs_time_apply(lfx_mrhs* m, const float* x, float* y, int32_t reps, float* us);
-/* apply autotuner: times 2, 4 and 8 levels per shared-memory block (those
- * that fit) over reps applies and keeps the fastest; outputs (nullable) the
- * choice and its time per apply in microseconds */
+/* times the apply over reps applies; outputs (nullable) the rows it holds at
+ * once and its time per apply in microseconds */
 int lfx_mrhs_autotune(lfx_mrhs* m, int32_t reps, int32_t* levels_per_block, float* us);
 enum { LFX_MRHS_PER_RHS_CG = 0, LFX_MRHS_BLOCK_CG = 1 };
 typedef struct {

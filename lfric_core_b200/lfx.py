@@ -518,9 +518,10 @@ def fem_operators(ctx, mesh, space, coef, precisions=(R64, R32)):
 
 
 class MultiRhsOperator(_Handle):
-    """One LMA operator applied to nrhs right-hand sides at once, the per-cell
-    products on the tensor cores (lfx_mrhs). Vectors are device arrays of
-    undf x nrhs FP32 values, dof-major, passed as device pointers (ints)."""
+    """One LMA operator applied to nrhs right-hand sides at once in FP32, from
+    column stencils summed once from its local matrices (lfx_mrhs). Vectors are
+    device arrays of undf x nrhs FP32 values, dof-major, passed as device
+    pointers (ints); kind is the least precision the caller takes."""
 
     _destroy = "lfx_mrhs_destroy"
 
@@ -567,7 +568,7 @@ class MultiRhsOperator(_Handle):
 
     def solve(self, op64: "LmaOperator", diag: "FieldVector", b_ptr: int, x_ptr: int, ld: int,
               r_tol=1e-8, inner_tol=1e-2, max_outer=20, max_inner=5000, method=MRHS_PER_RHS_CG):
-        """FP64 refinement around the FP32 tensor-core CG for all right-hand
+        """FP64 refinement around the FP32 CG for all right-hand
         sides (method: MRHS_PER_RHS_CG, or MRHS_BLOCK_CG for 64 right-hand
         sides); b, x: device FP64 arrays, right-hand side r at offset r * ld.
         Returns one SolveInfo per right-hand side."""

@@ -218,3 +218,42 @@ def test_block_cg_gram_products_match_fp64(ctx, nv):
         assert np.array_equal(got[0], got[1]), tensor
         G = np.concatenate(list(got[0]), axis=1)  # 64 x 64 nv
         assert np.all(np.abs(G - want) <= bound), (tensor, float(np.max(np.abs(G - want) / bound)))
+
+
+@pytest.mark.parametrize("n,nl,nrhs,patch,bits", [
+    (2, 1, 64, 0, 64), (3, 6, 16, 0, 64), (4, 7, 32, 5, 64), (5, 8, 64, 3, 32), (6, 11, 16, 0, 32),
+    (4, 16, 64, 40, 64), (9, 3, 32, 0, 64)])
+def test_mrhs_stencil_apply_is_fp32_accurate(ctx, n, nl, nrhs, patch, bits):
+    """Rows in groups of eight (heights 2 to 17), columns with three and four
+    cells around them, partial blocks. Each coefficient is rounded once from
+    its FP64 sum (FP32 operators: each cell's entry before that), then at most
+    27 FMAs: within 32 u |A| |x|, u = 2^-24, of the FP64 product."""
+    p = mg.w0_problem(n, nl, seed=31 + n)
+    s = wl.device_w0(ctx, p)
+    op = s.op if bits == 64 else s.op.like(p.lma, lfx.R32)
+    M = lfx.MultiRhsOperator(op, TF32, nrhs, patch)
+    X = np.random.default_rng(n).standard_normal((p.undf, nrhs)).astype(np.float32)
+    Y = mrhs_apply(ctx, M, X)
+    o, oa = o_lma(p), o_lma(p, np.abs(p.lma))
+    for r in range(0, nrhs, 5):
+        x = X[:, r].astype(np.float64)
+        assert np.all(np.abs(Y[:, r] - o.apply(x)) <= 32 * 2.0 ** -24 * oa.apply(np.abs(x)))
+
+
+def test_mrhs_apply_alignment(ctx):
+    p = mg.w0_problem(4, 5, seed=2)
+    s = wl.device_w0(ctx, p)
+    M = lfx.MultiRhsOperator(s.op, TF32, 16)
+    big = torch.randn(p.undf * 16 + 4, device="cuda")
+    y, z = torch.empty(p.undf * 16, device="cuda"), torch.empty(p.undf * 16, device="cuda")
+    x = big[2:2 + p.undf * 16]  # 8-byte aligned
+    aligned = x.clone()
+    torch.cuda.synchronize()
+    M.apply(x.data_ptr(), y.data_ptr())
+    M.apply(aligned.data_ptr(), z.data_ptr())
+    ctx.synchronize()
+    assert torch.equal(y, z)
+    for bad in ((aligned.data_ptr() + 4, y.data_ptr()), (aligned.data_ptr(), y.data_ptr() + 8)):
+        with pytest.raises(lfx.LfxError) as e:
+            M.apply(*bad)
+        assert e.value.status == 4
