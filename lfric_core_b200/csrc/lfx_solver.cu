@@ -20,6 +20,7 @@
 
 #include <type_traits>
 
+#include "lfx_cg_persist.cuh"
 #include "lfx_internal.cuh"
 
 namespace lfx {
@@ -555,6 +556,130 @@ int norm_kernel(lfx_ctx* ctx, int64_t n, const T* v, double* out, const int* ski
 }
 
 // ------------------------------------------------------------------ CG
+// The persistent form of the solve (lfx_cg_persist.cuh): blocks of a launch, 0
+// where the launch per phase is taken
+struct CgShape {
+  int grid = 0, lw = 5;
+  bool cluster = false;
+  // a second record's x value may have to come from outside its lanes: columns
+  // of more than 32 rows, or records that are not one level apart
+  bool edge = false;
+};
+
+CgShape cg_shape(const lfx_solver* s) {
+  const lfx_ctx* ctx = s->ctx;
+  const lfx_lma_layout* L = s->op->lay;
+  CgShape q;
+  // (per-apply events and a forced apply kernel need the launch per phase)
+  if (s->prec->kind != PREC_DIAG || ctx->time_applies || ctx->lma_kernel >= 0) return q;
+  if (!L->full_cover || !L->ent_pack || L->max_nrec > 2 || (L->ndf_from != 6 && L->ndf_from != 8))
+    return q;
+  // Up to a matrix the size of L2, which the gather rereads: C48 x 30 FP32 (106
+  // MB) 46.7 us an iteration by launches, 35.7 here; FP64 (212 MB) 67.5 and 66.8,
+  // and 54 by launches of the cell scatter.
+  if (s->op->mat_bytes > (size_t)ctx->l2_bytes) return q;
+  const int64_t nch = nchunks(s->n);
+  if (nch < 1 || nch > (int64_t)kCgSubs * ctx->num_sms) return q;
+  while (q.lw > 3 && L->max_h <= 1 << (q.lw - 1)) --q.lw;
+  q.edge = L->max_h > 32 || !L->cs_ok;  // (the scatter plan pairs consecutive levels only)
+  const int cols = 32 >> q.lw;  // of a warp
+  const int64_t warps = (L->nent + cols - 1) / cols, all = kCgThreads / 32;
+  q.cluster = warps <= kCgCluster * all && nch <= (int64_t)kCgSubs * kCgCluster;
+  // half-full blocks before a second column a warp
+  q.grid = q.cluster ? kCgCluster
+                     : (int)std::min<int64_t>(std::max((nch + kCgSubs - 1) / kCgSubs,
+                                                       (warps + all / 2 - 1) / (all / 2)),
+                                              ctx->num_sms);
+  return q;
+}
+
+template <class T, int N, bool CLUSTER, bool EDGE>
+int cg_persist_launch(lfx_ctx* ctx, CgArgs<T> A, DevState* S, const DevState& init, int first,
+                      int grid) {
+  auto kern = cg_persist<T, N, CLUSTER, EDGE, DevState>;
+  // a block's chunks, and its columns up to what a block may have
+  const size_t vec = (size_t)((A.nch + grid - 1) / grid) * cg_chunk_bytes<T>();
+  const size_t per = 32 >> A.lw, cols = ((size_t)(A.nent + grid - 1) / grid + per - 1) / per * per;
+  A.smem = (int)std::min(kCgSmemMax, vec + cols * A.maxg * cg_group_bytes<T, N>(A.nl));
+  static bool attr = false;
+  if (!attr) {
+    LFX_CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kCgSmemMax));
+    if (CLUSTER)
+      LFX_CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    attr = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kCgThreads);
+  cfg.dynamicSmemBytes = (size_t)A.smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  if (CLUSTER) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)grid;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    LFX_CK(ctx, cudaMemsetAsync(A.bar, 0, sizeof(unsigned), ctx->stream));
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  LFX_CK(ctx, cudaLaunchKernelEx(&cfg, kern, A, S, init, first));
+  ctx->launches++;
+  return LFX_OK;
+}
+
+template <class T, int N>
+int cg_persist_form(lfx_ctx* ctx, const CgArgs<T>& A, DevState* S, const DevState& init, int first,
+                    const CgShape& q) {
+  if (q.edge)
+    return q.cluster ? cg_persist_launch<T, N, true, true>(ctx, A, S, init, first, q.grid)
+                     : cg_persist_launch<T, N, false, true>(ctx, A, S, init, first, q.grid);
+  return q.cluster ? cg_persist_launch<T, N, true, false>(ctx, A, S, init, first, q.grid)
+                   : cg_persist_launch<T, N, false, false>(ctx, A, S, init, first, q.grid);
+}
+
+// the whole solve
+template <class T>
+int cg_run_persist(lfx_solver* s, const CgShape& q, T* x, const T* b) {
+  lfx_ctx* ctx = s->ctx;
+  const lfx_lma_layout* L = s->op->lay;
+  CgArgs<T> A{};
+  A.nent = L->nent;
+  A.nl = L->nlayers;
+  A.blk = s->op->blk;
+  A.gp_stride = L->gp_stride;
+  A.cell_stride = (size_t)L->ndf_to * s->op->blk;
+  A.ent_pack = L->ent_pack;
+  A.grp_pack = L->grp_pack;
+  A.M = (const T*)s->op->mat;
+  A.n = s->n;
+  A.nch = (int)nchunks(s->n);
+  A.x = x;
+  A.b = b;
+  A.r = (T*)s->work[0];
+  A.p = (T*)s->work[1];
+  A.z = (T*)s->work[2];
+  A.dg = (const T*)s->prec->rdiag;
+  A.partials = ctx->d_partials;
+  A.bar = ctx->d_ticket + 1;
+  A.err = ctx->d_err;
+  A.iters = kCgItersPerLaunch;
+  A.maxg = L->max_groups;
+  A.lw = q.lw;
+  for (int first = 1;; first = 0) {
+    const DevState init = *s->h_state;  // (as init_state left it, for the first launch)
+    int rc = L->ndf_from == 6 ? cg_persist_form<T, 6>(ctx, A, s->d_state, init, first, q)
+                              : cg_persist_form<T, 8>(ctx, A, s->d_state, init, first, q);
+    if (!rc) rc = read_state(s);
+    // a barrier that ran out leaves the state as it was
+    if (!rc && !s->h_state->done) rc = lfx_ctx_check_device_error(ctx);
+    if (rc || s->h_state->done) return rc;
+  }
+}
+
 template <class T>
 int cg_run(lfx_solver* s, T* x, const T* b) {
   lfx_ctx* ctx = s->ctx;
@@ -565,6 +690,8 @@ int cg_run(lfx_solver* s, T* x, const T* b) {
   T* z = (T*)s->work[2];
   const int* done = &S->done;
   int rc;
+  const CgShape shape = cg_shape(s);
+  if (shape.grid) return cg_run_persist<T>(s, shape, x, b);
   // r = b - A x   (apply, scale(-1), axpy(1, b): one rounding, b - Ax)
   if ((rc = op_apply_impl(s->op, x, r, b, nullptr))) return rc;
   rc = launch_chunks<1>(
@@ -1486,8 +1613,7 @@ int lfx_solver_apply(lfx_solver* s, lfx_vec* x, const lfx_vec* b, lfx_solve_info
       rc = s->precision == LFX_R64
                ? gmres_run<double>(s, (double*)x->data[0], (const double*)b->data[0])
                : gmres_run<float>(s, (float*)x->data[0], (const float*)b->data[0]);
-    if (!rc) rc = read_state(s);
-    if (!rc) fill_info(s, info);
+    if (!rc) fill_info(s, info);  // (each of them ends with the state read)
   }
   if (ctx->time_applies) drain_timing(ctx);
   if (!rc) rc = lfx_ctx_check_device_error(ctx);
