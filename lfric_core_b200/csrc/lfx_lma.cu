@@ -2192,6 +2192,8 @@ void launch_apply(lfx_ctx* ctx, const lfx_op* op, int kernel, const TmaShape& ts
     launch_apply_t<float>(ctx, op, kernel, ts, x, y, b, skip);
 }
 
+constexpr size_t kCellsMinBytes = (size_t)24 << 20;
+
 // the configuration an apply of this operator uses
 void pick_apply(const lfx_ctx* ctx, const lfx_op* op, int* kernel, TmaShape* ts) {
   *ts = TmaShape{};
@@ -2235,8 +2237,20 @@ void pick_apply(const lfx_ctx* ctx, const lfx_op* op, int* kernel, TmaShape* ts)
     }
     if ((*kernel != 0 && *kernel != 4) || ts->warps) return;
   }
-  // untuned: the prefetching gather where it fits (fastest measured on W2
-  // and W3 columns), else the register gather, else the generic one
+  // untuned, a symmetric operator of some size: the cell scatter, which reads
+  // the packed triangle (each entry once) where the gathers read the whole
+  // matrix. Its launch per colour costs 9 to 13 us by itself, so the line is at
+  // a 24 MB matrix. Prefetching / register gather and cell scatter in us: W0
+  // FP64 C16 x 10 (8 MB) 8.3, 13.0; C24 x 20 (35 MB) 16.5, 13.7; C48 x 30 (212
+  // MB) 48.3, 36.9; W0 FP32 C24 x 20 (18 MB) 10.4, 12.4; C37 x 23 (48 MB) 18.6,
+  // 16.5; W2 FP64 C24 x 20 (20 MB) 10.4, 10.3; C37 x 23 (54 MB) 18.6, 16.5; W2
+  // FP32 C37 x 23 (28 MB) 13.6, 13.4; C48 x 30 (60 MB) 20.6, 16.4.
+  if (cells_ok(op) && op->smat && op->mat_bytes >= kCellsMinBytes) {
+    *kernel = 5;
+    return;
+  }
+  // else the prefetching gather where it fits, the register gather, the
+  // generic one
   *kernel = fetch_ok(op) ? 3 : (gather2_ok(op) ? 1 : 2);
 }
 
