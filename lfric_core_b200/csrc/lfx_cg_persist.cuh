@@ -43,7 +43,7 @@ struct CgArgs {
   T *x, *r, *p, *z;
   const T* dg;
   double* partials;  // 3 nch
-  unsigned* bar;     // arrivals, zero at launch
+  unsigned* bar;     // {arrivals, blocks gone}, zero between launches
   int* err;
   int iters;
   const T* b;
@@ -103,6 +103,14 @@ __device__ __forceinline__ bool cg_barrier(unsigned* bar, int* err, unsigned& ta
     }
     __syncthreads();
     return *ok != 0;
+  }
+}
+
+// the last block to leave makes the barrier ready for the next launch
+__device__ __forceinline__ void cg_leave(unsigned* bar) {
+  if (threadIdx.x == 0 && atomicAdd(bar + 1, 1u) == gridDim.x - 1) {
+    bar[0] = 0u;
+    bar[1] = 0u;
   }
 }
 
@@ -468,6 +476,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_persist(CgArgs<T> A, State* 
     A.r[base + m * RT] = rs[m * RT + tid];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *S = c;
+  if (!CLUSTER) cg_leave(A.bar);
 }
 
 }  // namespace lfx

@@ -243,8 +243,9 @@ int lfx_ctx_check_device_error(lfx_ctx* ctx) {
   LFX_CK(ctx, cudaStreamSynchronize(ctx->stream));
   LFX_CK(ctx, cudaMemcpy(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (h) {
-    // the flag, and the grid barrier words of a persistent apply that left early
+    // the flag, and the grid barrier words of a persistent launch that left early
     LFX_CK(ctx, cudaMemset(ctx->d_err, 0, sizeof(int) * 4));
+    LFX_CK(ctx, cudaMemset(ctx->d_ticket + 1, 0, sizeof(unsigned) * 2));
     return fail(ctx, LFX_TIMEOUT, "a device-side bounded wait ran out (pipeline stage never filled)");
   }
   return LFX_OK;

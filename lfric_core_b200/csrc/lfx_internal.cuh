@@ -33,7 +33,7 @@ struct lfx_ctx {
   // reduction scratch: partials of up to 4 simultaneous sums, one ticket
   double* d_partials = nullptr;
   int64_t partials_cap = 0;  // doubles
-  unsigned* d_ticket = nullptr;  // [0] of the reductions, [1] arrivals of the persistent CG
+  unsigned* d_ticket = nullptr;  // [0] of the reductions, [1..2] barrier of the persistent solver launches
   // small device scratch for scalar results of the C-ABI reductions
   double* d_scalars = nullptr;
   double* h_scalars = nullptr;      // pinned, mapped into the device's address space

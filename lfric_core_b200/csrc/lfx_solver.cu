@@ -22,6 +22,7 @@
 
 #include "lfx_cg_persist.cuh"
 #include "lfx_internal.cuh"
+#include "lfx_mgs_persist.cuh"
 
 namespace lfx {
 int drain_timing(lfx_ctx* ctx);
@@ -30,7 +31,7 @@ using namespace lfx;
 
 namespace {
 
-constexpr int MAX_GCRK = 64;
+constexpr int MAX_GCRK = kMgsMaxVec;
 constexpr double EPS_RDEF = DBL_EPSILON;  // constants_mod.F90:167
 
 struct DevState {
@@ -622,7 +623,6 @@ int cg_persist_launch(lfx_ctx* ctx, CgArgs<T> A, DevState* S, const DevState& in
   } else {
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
-    LFX_CK(ctx, cudaMemsetAsync(A.bar, 0, sizeof(unsigned), ctx->stream));
   }
   cfg.attrs = at;
   cfg.numAttrs = 1;
@@ -982,6 +982,32 @@ __global__ void __launch_bounds__(256) gmres_xupdate(int64_t n, VecPtrs vp, cons
   }
 }
 
+template <class T>
+int mgs_launch(lfx_ctx* ctx, const MgsArgs<T>& A) {
+  static bool attr = false;
+  if (!attr) {
+    LFX_CK(ctx, cudaFuncSetAttribute(mgs_persist<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kMgsSmemMax));
+    attr = true;
+  }
+  // a chunk a sub-group while there are blocks for it
+  const int grid = std::max(1, std::min((A.nch + kCgSubs - 1) / kCgSubs, ctx->num_sms));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(kCgThreads);
+  cfg.dynamicSmemBytes =
+      std::min<size_t>(kMgsCap<T>, (size_t)(A.nch + grid - 1) / grid) * RCHUNK * sizeof(T);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  LFX_CK(ctx, cudaLaunchKernelEx(&cfg, mgs_persist<T>, A));
+  ctx->launches++;
+  return LFX_OK;
+}
+
 // sig (nullable): scales of an unnormalised basis, folded into u
 __global__ void gmres_finish_cycle(DevState* S, double* gm, int K, const double* sig,
                                    int count_cycle) {
@@ -1159,6 +1185,25 @@ int gmres_run(lfx_solver* s, T* x, const T* b, bool one_cycle = false) {
         for (int k = 0; k < iv; ++k) vpi.p[k] = V[k];
         q = cgs_step<T>(ctx, n, iv, vpi, w, col, &nh[(K + 1) * (iv - 1)], fin_norm, askip);
         if (q) return q;
+      } else if (!s->inner_mode) {
+        MgsArgs<T> A{};
+        A.n = n;
+        A.nch = (int)nchunks(n);
+        A.iv = iv;
+        for (int k = 0; k < iv; ++k) A.v[k] = V[k];
+        A.w = w;
+        A.vn = iv < K ? V[iv] : nullptr;
+        A.h = col;
+        A.nh = &nh[(K + 1) * (iv - 1)];
+        A.inv_hn = &S->inv_hn;
+        A.sig = &sig[iv];
+        A.applies = &S->applies;
+        A.partials = ctx->d_partials;
+        A.bar = ctx->d_ticket + 1;
+        A.err = ctx->d_err;
+        A.skip = askip;
+        if ((q = mgs_launch(ctx, A))) return q;
+        continue;
       } else {
       // modified Gram-Schmidt (the reference's): h(j,iv) = <v_j, w> ; w -= h(j,iv) v_j
       {
