@@ -666,23 +666,28 @@ constexpr size_t tc_gram_smem() {
 }
 
 // out[e] = sum over the blocks, in block order, of partials[b][e]
-__global__ void bcg_reduce(int nb, int ne, const double* __restrict__ partials,
-                           double* __restrict__ out, const BcgSmall* st) {
+// A block takes 32 entries, warp w the w-th eighth of the partials; the eight
+// sums are added left to right. (One thread an entry, 16 blocks in all for a
+// Gram, took 28 us of 296 x 32 KB.)
+__global__ void __launch_bounds__(256) bcg_reduce(int nb, int ne,
+                                                  const double* __restrict__ partials,
+                                                  double* __restrict__ out, const BcgSmall* st) {
+  __shared__ double sm[8][32];
   if (st->done) return;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  // block order, as before; eight loads in flight ahead of the additions
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int e = blockIdx.x * 32 + lane;
+  const int b0 = nb * w / 8, b1 = nb * (w + 1) / 8;
   double s = 0.0;
-  int b = 0;
-  for (; b + 8 <= nb; b += 8) {
-    double v[8];
+#pragma unroll 8
+  for (int b = b0; b < b1; ++b)
+    if (e < ne) s = s + __ldg(partials + (size_t)b * ne + e);
+  sm[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && e < ne) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = __ldg(partials + (size_t)(b + q) * ne + e);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) s = s + v[q];
+    for (int q = 1; q < 8; ++q) s = s + sm[q][lane];
+    out[e] = s;
   }
-  for (; b < nb; ++b) s = s + __ldg(partials + (size_t)b * ne + e);
-  out[e] = s;
 }
 
 // ---- The same products with the tall blocks streamed. A block takes the
@@ -1020,57 +1025,115 @@ __global__ void __launch_bounds__(256) bcg_mask(int64_t n, float* R, const int* 
 //   right-hand side has rn <= tol r0); beta = -L1^T (L1 Q^T D^-1 R)
 // mode 2 (orth): pivoted Cholesky of W^T W -> rank and T (P = W T)
 // mode 3 (norms of the initial residual into r0)
+//
+// Both factorisations run as one elimination of [G | I] in registers: 256
+// threads hold 4 x 4 entries of each half (rows tr + 16 a, columns tc + 16 b of
+// thread 16 tr + tc), and a step subtracts multiples of the pivot's row, passed
+// round through shared memory, from the rows not yet eliminated; their column of
+// the pivot is that row by symmetry. The left half ends as D L^T and the right
+// one, its rows scaled by 1 / sqrt(d), as L^-1, with no substitution after it.
+// One barrier a step, with pivoting too: every warp keeps the diagonal, which
+// the pivot's row updates. A form
+// that factorised in shared memory, entry by entry, and then substituted took 88
+// us (mode 0), 25 us (mode 1) and 129 us (mode 2); this one 31, 15 and 42: the
+// chain of a step (row, division, products, barrier) is 0.4 to 0.6 us.
+//
 // The kernel's whole shared state is one dynamic buffer laid out here (no
-// static shared variables beside it): three 64 x 65 FP64 matrices, then the
-// pivot order and two flags.
+// static shared variables beside it): three 64 x 65 FP64 matrices, the pivot's
+// row (two buffers), the pivots, then the step of each row.
 constexpr size_t kBcgMatBytes = sizeof(double) * kBS * (kBS + 1);
-constexpr size_t kBcgSmallSmem = 3 * kBcgMatBytes + sizeof(int) * (kBS + 4);
+constexpr size_t kBcgSmallSmem =
+    3 * kBcgMatBytes + sizeof(double) * (4 * kBS + kBS) + sizeof(int) * kBS;
 
-// Linv = L^-1 for the r x r lower factor L(i, k): thread j < r forms column
-// j (rows below j by forward substitution, the dot products in four partial
-// sums); rows and columns past r are zero
-template <class Lf>
-__device__ __forceinline__ void lower_inverse(int r, Lf L, double (*Linv)[kBS + 1]) {
-  const int t = threadIdx.x;
-  if (t < kBS) {
-    const int j = t;
-    for (int i = 0; i < kBS; ++i) Linv[i][j] = 0.0;
-    if (j < r) {
-      Linv[j][j] = 1.0 / L(j, j);
-      for (int i = j + 1; i < r; ++i) {
-        double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
-        int k = j;
-        for (; k + 3 < i; k += 4) {
-          v0 = fma(L(i, k), Linv[k][j], v0);
-          v1 = fma(L(i, k + 1), Linv[k + 1][j], v1);
-          v2 = fma(L(i, k + 2), Linv[k + 2][j], v2);
-          v3 = fma(L(i, k + 3), Linv[k + 3][j], v3);
-        }
-        for (; k < i; ++k) v0 = fma(L(i, k), Linv[k][j], v0);
-        Linv[i][j] = -((v0 + v1) + (v2 + v3)) / L(i, i);
+// this thread's entries of [G | I] (I: the first r rows)
+struct BcgElim {
+  double A[4][4], B[4][4];
+  int tr, tc;
+  __device__ __forceinline__ void load(const double* G, int r) {
+    tr = threadIdx.x >> 4;
+    tc = threadIdx.x & 15;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int i = tr + 16 * a, j = tc + 16 * b;
+        A[a][b] = G[i * kBS + j];
+        B[a][b] = i == j && i < r ? 1.0 : 0.0;
       }
+  }
+  // row p into R[0 .. 64) and R[64 .. 128)
+  __device__ __forceinline__ void put(int p, double* R) const {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if (tr + 16 * a == p) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          R[tc + 16 * b] = A[a][b];
+          R[kBS + tc + 16 * b] = B[a][b];
+        }
+      }
+  }
+  // the rows of `rest` lose their multiple of row R: row groups A0 .. 3, of the
+  // left half the columns of the same groups and of the right one those of
+  // groups 0 .. B1
+  template <int A0, int B1>
+  __device__ __forceinline__ void sub(const double* R, double inv, unsigned long long rest) {
+    double ra[4], rb[4];
+#pragma unroll
+    for (int b = A0; b < 4; ++b) ra[b] = R[tc + 16 * b];
+#pragma unroll
+    for (int b = 0; b <= B1; ++b) rb[b] = R[kBS + tc + 16 * b];
+    rest >>= tr;
+#pragma unroll
+    for (int a = A0; a < 4; ++a) {
+      const double m = (rest >> (16 * a)) & 1ull ? -(R[tr + 16 * a] * inv) : 0.0;
+      if (m == 0.0) continue;
+#pragma unroll
+      for (int b = A0; b < 4; ++b) A[a][b] = fma(m, ra[b], A[a][b]);
+#pragma unroll
+      for (int b = 0; b <= B1; ++b) B[a][b] = fma(m, rb[b], B[a][b]);
     }
   }
-  __syncthreads();
-}
+  // steps 16 KA .. of the unpivoted elimination; false when a pivot is not positive
+  template <int KA>
+  __device__ __forceinline__ bool steps(int r, unsigned long long upto, double* row, double* piv) {
+    for (int k = 16 * KA; k < min(r, 16 * KA + 16); ++k) {
+      double* R = row + (k & 1) * 2 * kBS;
+      if (tr == k - 16 * KA) {
+#pragma unroll
+        for (int b = KA; b < 4; ++b) R[tc + 16 * b] = A[KA][b];
+#pragma unroll
+        for (int b = 0; b <= KA; ++b) R[kBS + tc + 16 * b] = B[KA][b];
+      }
+      __syncthreads();
+      const double d = R[k];
+      if (!(d > 0.0)) return false;  // every thread reads the same d
+      if (threadIdx.x == 0) piv[k] = d;
+      sub<KA, KA>(R, 1.0 / d, k == 63 ? 0ull : upto & (~0ull << (k + 1)));
+    }
+    return true;
+  }
+};
 
-// Out = op(A) B for 64 x 64 operands, op(A) = A or A^T; each thread a 4 x 4
-// tile, k in increasing order
+// Out = op(A) B for 64 x 64 operands, op(A) = A or A^T; each thread the 4 x 4
+// entries (tr + 16 x, tc + 16 y), so that the 16 threads of a row read 16
+// neighbouring columns of B; k in increasing order
 template <bool TRANS>
 __device__ __forceinline__ void small_mm(const double (*A)[kBS + 1], const double (*B)[kBS + 1],
                                          double (*Out)[kBS + 1], double scale) {
-  const int i0 = 4 * (threadIdx.x / 16), j0 = 4 * (threadIdx.x % 16);
+  const int tr = threadIdx.x / 16, tc = threadIdx.x % 16;
   double acc[4][4];
 #pragma unroll
   for (int x = 0; x < 4; ++x)
 #pragma unroll
     for (int y = 0; y < 4; ++y) acc[x][y] = 0.0;
+#pragma unroll 4
   for (int k = 0; k < kBS; ++k) {
     double a[4], bv[4];
 #pragma unroll
-    for (int x = 0; x < 4; ++x) a[x] = TRANS ? A[k][i0 + x] : A[i0 + x][k];
+    for (int x = 0; x < 4; ++x) a[x] = TRANS ? A[k][tr + 16 * x] : A[tr + 16 * x][k];
 #pragma unroll
-    for (int y = 0; y < 4; ++y) bv[y] = B[k][j0 + y];
+    for (int y = 0; y < 4; ++y) bv[y] = B[k][tc + 16 * y];
 #pragma unroll
     for (int x = 0; x < 4; ++x)
 #pragma unroll
@@ -1080,7 +1143,7 @@ __device__ __forceinline__ void small_mm(const double (*A)[kBS + 1], const doubl
 #pragma unroll
   for (int x = 0; x < 4; ++x)
 #pragma unroll
-    for (int y = 0; y < 4; ++y) Out[i0 + x][j0 + y] = scale * acc[x][y];
+    for (int y = 0; y < 4; ++y) Out[tr + 16 * x][tc + 16 * y] = scale * acc[x][y];
   __syncthreads();
 }
 
@@ -1089,9 +1152,9 @@ __global__ void __launch_bounds__(256) bcg_small(int mode, BcgSmall* st, double 
   double (*M)[kBS + 1] = reinterpret_cast<double (*)[kBS + 1]>(bcg_dyn);
   double (*Bm)[kBS + 1] = reinterpret_cast<double (*)[kBS + 1]>(bcg_dyn + kBcgMatBytes);
   double (*Y)[kBS + 1] = reinterpret_cast<double (*)[kBS + 1]>(bcg_dyn + 2 * kBcgMatBytes);
-  int* perm = reinterpret_cast<int*>(bcg_dyn + 3 * kBcgMatBytes);
-  int& s_r = perm[kBS];
-  int& s_stop = perm[kBS + 1];
+  double* row = reinterpret_cast<double*>(bcg_dyn + 3 * kBcgMatBytes);  // [2][2 kBS]
+  double* piv = row + 4 * kBS;
+  int* pos = reinterpret_cast<int*>(piv + kBS);
   const int t = threadIdx.x;
   if (st->done) return;
   if (mode == 3) {
@@ -1105,142 +1168,111 @@ __global__ void __launch_bounds__(256) bcg_small(int mode, BcgSmall* st, double 
   if (mode == 0 || mode == 1) {
     const int r = st->rank;
     if (mode == 0) {
-      // Cholesky of the r x r active block of P^T Q (column by column)
-      for (int e = t; e < kBS * kBS; e += blockDim.x) M[e / kBS][e % kBS] = st->C[e];
-      __syncthreads();
-      // two barriers a step: every thread takes the pivot's root from the
-      // diagonal itself (written back only in the update phase, which does
-      // not read it), the column is divided, then the trailing triangle is
-      // updated by a 16 x 16 thread grid (no index division)
-      const int ti = t >> 4, tj = t & 15;
-      bool stop = false;
-      for (int k = 0; k < r; ++k) {
-        const double d = M[k][k];
-        if (!(d > 0.0)) {
-          stop = true;  // every thread reads the same d
-          break;
-        }
-        const double sk = sqrt(d);
-        for (int i = k + 1 + t; i < r; i += blockDim.x) M[i][k] /= sk;
-        __syncthreads();
-        if (t == 0) M[k][k] = sk;
-        for (int i = k + 1 + ti; i < r; i += 16) {
-          const double lik = M[i][k];
-          for (int j = k + 1 + tj; j <= i; j += 16) M[i][j] -= lik * M[j][k];
-        }
-        __syncthreads();
-      }
+      // elimination of the r x r active block of P^T Q
+      BcgElim e;
+      e.load(st->C, r);
+      const unsigned long long upto = r == 64 ? ~0ull : (1ull << r) - 1ull;
+      const bool stop = !(e.steps<0>(r, upto, row, piv) && e.steps<1>(r, upto, row, piv) &&
+                          e.steps<2>(r, upto, row, piv) && e.steps<3>(r, upto, row, piv));
       if (stop) {
         if (t == 0) { st->fail = 1; st->done = 1; }
         return;
       }
-      // L1 = L^-1, kept for mode 1
-      lower_inverse(r, [&](int i, int k) { return M[i][k]; }, Bm);
-      for (int e = t; e < kBS * kBS; e += blockDim.x) st->L1[e] = Bm[e / kBS][e % kBS];
-      // right-hand sides: P^T R
-      for (int e = t; e < kBS * kBS; e += blockDim.x) M[e / kBS][e % kBS] = st->C[kBS * kBS + e];
       __syncthreads();
+      // L1 = L^-1, kept for mode 1; rows and columns past r are zero
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const int i = e.tr + 16 * a;
+        const double sc = i < r ? 1.0 / sqrt(piv[i]) : 0.0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const double v = i < r ? e.B[a][b] * sc : 0.0;
+          Bm[i][e.tc + 16 * b] = v;
+          st->L1[i * kBS + e.tc + 16 * b] = v;
+        }
+      }
+      // right-hand sides: P^T R; rows past r do not take part
+      for (int q = t; q < kBS * kBS; q += blockDim.x)
+        M[q / kBS][q % kBS] = q / kBS < r ? st->C[kBS * kBS + q] : 0.0;
     } else {
-      if (t < kBS) st->rn[t] = sqrt(st->rn[t]);
-      __syncthreads();
+      int over = 0;
+      if (t < kBS) {
+        const double rn = sqrt(st->rn[t]);
+        st->rn[t] = rn;
+        over = st->active[t] && rn > tol * st->r0[t];
+      }
+      const int go_on = __syncthreads_or(over);
       if (t == 0) {
-        int done = 1;
-        for (int j = 0; j < kBS; ++j)
-          if (st->active[j] && st->rn[j] > tol * st->r0[j]) done = 0;
         st->iters += 1;
-        s_stop = done;
+        if (!go_on) st->done = 1;
       }
-      __syncthreads();
-      if (s_stop) {
-        if (t == 0) st->done = 1;
-        return;
+      if (!go_on) return;
+      for (int q = t; q < kBS * kBS; q += blockDim.x) {
+        Bm[q / kBS][q % kBS] = st->L1[q];
+        M[q / kBS][q % kBS] = q / kBS < r ? st->E[q] : 0.0;
       }
-      for (int e = t; e < kBS * kBS; e += blockDim.x) {
-        Bm[e / kBS][e % kBS] = st->L1[e];
-        M[e / kBS][e % kBS] = st->E[e];
-      }
-      __syncthreads();
     }
-    // rows past r of the right-hand sides do not take part
-    for (int e = t; e < kBS * kBS; e += blockDim.x)
-      if (e / kBS >= r) M[e / kBS][e % kBS] = 0.0;
     __syncthreads();
     // Y = L1 B, then the coefficients L1^T Y (negated for beta)
     small_mm<false>(Bm, M, Y, 1.0);
     small_mm<true>(Bm, Y, Y, mode == 0 ? 1.0 : -1.0);
-    for (int e = t; e < kBS * kBS; e += blockDim.x) st->coef[e] = (float)Y[e / kBS][e % kBS];
+    for (int q = t; q < kBS * kBS; q += blockDim.x) st->coef[q] = (float)Y[q / kBS][q % kBS];
     return;
   }
-  // mode 2: pivoted Cholesky of G = W^T W, stopping at pivots below
-  // kBcgDrop times the largest diagonal entry. The pivoting is by index:
-  // rows and columns stay where they are and perm[i] names the row of step
-  // i, so L[i][j] = M[perm[i]][perm[j]] (i >= j) once the loop is done. (A
-  // form that swapped rows and columns in place, in one thread inside the
-  // loop over steps, lost the pivot's square root on the B200 while the same
-  // statements with a constant step index did not; the index form has no
-  // such swaps.) Warp 0 finds each pivot: the largest remaining diagonal
-  // entry, the first in step order on a tie.
-  for (int e = t; e < kBS * kBS; e += blockDim.x) M[e / kBS][e % kBS] = st->G[e];
-  if (t < kBS) perm[t] = t;
-  if (t == 0) s_r = 0;
-  __syncthreads();
+  // mode 2: pivoted elimination of G = W^T W, stopping at pivots below kBcgDrop
+  // times the first. Nothing is swapped: `rest` are the rows left and pos[i] the
+  // step that took row i. The pivot is the largest diagonal entry left to 14
+  // bits (the first of those that agree): its leading bits and its row make one
+  // 32-bit key for the warp's maximum. A row whose entry is not positive is none.
+  BcgElim e;
+  e.load(st->G, kBS);
+  const int lane = t & 31;
+  double dg[2] = {st->G[lane * (kBS + 1)], st->G[(lane + 32) * (kBS + 1)]};
+  unsigned long long rest = ~0ull;
+  int r = 0;
   double dmax = 0.0;
-  for (int i = 0; i < kBS; ++i) dmax = fmax(dmax, M[i][i]);
-  const int ti = t >> 4, tj = t & 15;
   for (int k = 0; k < kBS; ++k) {
-    if (t < 32) {
-      // lane l looks at steps k + l and k + l + 32
-      double bv = -INFINITY;
-      int bi = kBS;  // none (every candidate NaN): the factorisation stops
-      for (int i = k + t; i < kBS; i += 32) {
-        const double dv = M[perm[i]][perm[i]];
-        if (dv > bv) { bv = dv; bi = i; }
-      }
+    unsigned key = 0u;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-      }
-      if (t == 0) {
-        const int p = bi < kBS ? bi : k;
-        const int pk = perm[p];
-        const int stop = bi >= kBS || !(M[pk][pk] > kBcgDrop * dmax) || !(dmax > 0.0);
-        if (!stop) {
-          perm[p] = perm[k];
-          perm[k] = pk;
-          M[pk][pk] = sqrt(M[pk][pk]);
-          s_r = k + 1;
-        }
-        s_stop = stop;
-      }
+    for (int h = 0; h < 2; ++h) {
+      const int i = lane + 32 * h;
+      if (((rest >> i) & 1ull) && dg[h] > 0.0)
+        key = max(key, ((unsigned)__double2hiint(dg[h]) & ~63u) | (unsigned)(63 - i));
     }
-    __syncthreads();
-    if (s_stop) break;
-    const int pk = perm[k];
-    for (int i = k + 1 + t; i < kBS; i += blockDim.x) M[perm[i]][pk] /= M[pk][pk];
-    __syncthreads();
-    // the trailing square by a 16 x 16 thread grid (no index division)
-    const int m = kBS - k - 1;
-    for (int a = ti; a < m; a += 16) {
-      const int pi = perm[k + 1 + a];
-      const double lik = M[pi][pk];
-      for (int b = tj; b < m; b += 16) {
-        const int pj = perm[k + 1 + b];
-        M[pi][pj] -= lik * M[pj][pk];
-      }
+    key = __reduce_max_sync(0xffffffffu, key);
+    if (key < 64u) break;  // (the same in every thread, as below)
+    const int p = 63 - (int)(key & 63u);
+    const double d = __shfl_sync(0xffffffffu, p < 32 ? dg[0] : dg[1], p & 31);
+    if (k == 0) dmax = d;
+    if (!(d > kBcgDrop * dmax)) break;
+    double* R = row + (k & 1) * 2 * kBS;
+    e.put(p, R);
+    if (t == 0) {
+      piv[k] = d;
+      pos[p] = k;
     }
+    rest &= ~(1ull << p);
+    r = k + 1;
+    const double inv = 1.0 / d;
     __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const double x = R[lane + 32 * h];
+      dg[h] = fma(-(x * inv), x, dg[h]);
+    }
+    e.sub<0, 3>(R, inv, rest);
   }
-  const int r = s_r;
-  // Linv = L^-1 (r x r, lower; L[i][k] = M[perm[i]][perm[k]])
-  lower_inverse(r, [&](int i, int k) { return M[perm[i]][perm[k]]; }, Bm);
-  // T[perm[i]][j] = Linv[j][i] (i <= j < r), zero elsewhere
-  for (int e = t; e < kBS * kBS; e += blockDim.x) st->coef[e] = 0.f;
+  for (int q = t; q < kBS * kBS; q += blockDim.x) st->coef[q] = 0.f;
   __syncthreads();
-  for (int e = t; e < r * r; e += blockDim.x) {
-    const int i = e / r, j = e % r;
-    if (i <= j) st->coef[perm[i] * kBS + j] = (float)Bm[j][i];
+  // T(c, j) = L^-1(j, c), the step of a row naming its column of T
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int i = e.tr + 16 * a;
+    if ((rest >> i) & 1ull) continue;
+    const int j = pos[i];
+    const double sc = 1.0 / sqrt(piv[j]);
+#pragma unroll
+    for (int b = 0; b < 4; ++b) st->coef[(e.tc + 16 * b) * kBS + j] = (float)(e.B[a][b] * sc);
   }
   if (t == 0) {
     st->rank = r;
@@ -1765,7 +1797,7 @@ int gram(lfx_mrhs* m, const float* U, const float* V0, const float* V1, const fl
     bcg_gram_s<NV><<<m->bgrid, 256, smem, ctx->stream>>>(n, U, V0, V1, vscale, m->bpart, st);
   }
   const int ne = NV * kBS * kBS;
-  bcg_reduce<<<(ne + 255) / 256, 256, 0, ctx->stream>>>(m->bgrid, ne, m->bpart, out, st);
+  bcg_reduce<<<(ne + 31) / 32, 256, 0, ctx->stream>>>(m->bgrid, ne, m->bpart, out, st);
   ctx->launches += 2;
   LFX_CK(ctx, cudaGetLastError());
   return LFX_OK;
@@ -1821,7 +1853,7 @@ int bcg_inner(lfx_mrhs* m, const int* act, double tol, int max_inner, int* inner
   // r0: column norms of R (the update kernel's norm pass, products left out)
   upd_launch<0>(ctx, G)(n, m->p32, m->q32, m->x32, m->r32, m->dinv, st, 1,
                                             m->bpart);
-  bcg_reduce<<<1, kBS, 0, ctx->stream>>>(G, kBS, m->bpart, st->rn, st);
+  bcg_reduce<<<kBS / 32, 256, 0, ctx->stream>>>(G, kBS, m->bpart, st->rn, st);
   bcg_small<<<1, 256, kBcgSmallSmem, ctx->stream>>>(3, st, tol);
   // P = orth(D^-1 R)
   upd_launch<1>(ctx, G)(n, m->p32, m->r32, m->w32, nullptr, m->dinv, st, 1,
@@ -1833,8 +1865,10 @@ int bcg_inner(lfx_mrhs* m, const int* act, double tol, int max_inner, int* inner
                                             nullptr);
   ctx->launches += 10;
   LFX_CK(ctx, cudaGetLastError());
-  int it = 0;
-  while (it < max_inner) {
+  // four iterations between the host's looks at the state (every kernel but the
+  // apply idles once the solve is done)
+  constexpr int kCheck = 4;
+  for (int it = 1; it <= max_inner; ++it) {
     // Q = A P; alpha
     rc = mrhs_launch(m, m->p32, m->q32);
     if (!rc) rc = gram<2>(m, m->p32, m->q32, m->r32, nullptr, st, st->C);
@@ -1843,7 +1877,7 @@ int bcg_inner(lfx_mrhs* m, const int* act, double tol, int max_inner, int* inner
     // X += P alpha, R -= Q alpha, ||R_j||
     upd_launch<0>(ctx, G)(n, m->p32, m->q32, m->x32, m->r32, m->dinv, st, 0,
                                               m->bpart);
-    bcg_reduce<<<1, kBS, 0, ctx->stream>>>(G, kBS, m->bpart, st->rn, st);
+    bcg_reduce<<<kBS / 32, 256, 0, ctx->stream>>>(G, kBS, m->bpart, st->rn, st);
     // beta (and convergence)
     rc = gram<1>(m, m->q32, m->r32, nullptr, m->dinv, st, st->E);
     if (rc) return rc;
@@ -1858,7 +1892,7 @@ int bcg_inner(lfx_mrhs* m, const int* act, double tol, int max_inner, int* inner
                                               0, nullptr);
     ctx->launches += 13;
     LFX_CK(ctx, cudaGetLastError());
-    ++it;
+    if (it % kCheck && it < max_inner) continue;
     LFX_CK(ctx, cudaMemcpyAsync(&m->h_bcg->rank, &st->rank, 4 * sizeof(int),
                                 cudaMemcpyDeviceToHost, ctx->stream));
     LFX_CK(ctx, cudaStreamSynchronize(ctx->stream));
