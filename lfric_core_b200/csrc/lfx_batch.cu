@@ -35,9 +35,9 @@
 //   P   p = z + beta p
 // Work items: apply items of up to `cells_per_item` cell columns of one
 // colour of one slot, one warp each (a column's segments in order);
-// 16384-value chunk items (slot, chunk), one block each, for the vector
+// 4096-value chunk items (slot, chunk), one block each, for the vector
 // phases; 64-column items for the sweeps. Per-slot sums are reduced in an
-// order fixed by the slot alone (per cell column, per 16384-value chunk, then
+// order fixed by the slot alone (per cell column, per 4096-value chunk, then
 // in index order), so a slot's result is bit-identical whatever else is in
 // the batch and whatever launch shape the autotuner picks.
 //
@@ -65,7 +65,7 @@ constexpr double kDelta = 1e-3;  // reliable update when ||r|| drops by this fac
 constexpr int kBT = 256;         // threads per block of the persistent kernel
 constexpr int kBW = kBT / 32;    // warps per block
 constexpr int kMaxBps = 3;       // blocks per SM the kernel is built for (launch bounds)
-constexpr int kBSub = 8;         // a chunk item: kBSub chunks of RCHUNK values (16384)
+constexpr int kBSub = 2;         // a chunk item: kBSub chunks of RCHUNK values (4096)
 constexpr int kMaxIters = 64;    // super-iterations per launch, at most
 constexpr int kMaxSeg = 4;       // warps (segments of <= 31 levels) per cell column, at most
 constexpr int kMaxColours = 8;   // cell colours of a slot, at most
@@ -183,34 +183,35 @@ __device__ __forceinline__ unsigned atom_add_acqrel(unsigned* p, unsigned v) {
 // Grid-wide barrier of a cooperative launch. Thread 0 of each block reads the
 // generation, arrives, and the last to arrive resets the count and releases
 // the next generation; the others spin on it for at most timeout_ns (and stop
-// at once when another block has reported an error). Returns false when the
-// block must leave the kernel.
+// when another block has reported an error). Returns false when the block must
+// leave the kernel. (Pauses of 100 ns between polls and fences beside the
+// acquire and release cost 2 % of a small batch.)
 __device__ bool grid_sync(const BParams& P, BShared& sh) {
   __syncthreads();
   if (threadIdx.x == 0) {
     int ok = 1;
     const unsigned gen = ld_acquire(P.bar + 1);
-    __threadfence();
     const unsigned arrived = atom_add_acqrel(P.bar, 1u);
     if (arrived == gridDim.x - 1) {
       P.bar[0] = 0u;
       st_release(P.bar + 1, gen + 1u);
     } else {
-      const unsigned long long t0 = gtimer();
-      while (ld_acquire(P.bar + 1) == gen) {
+      unsigned long long t0 = 0;
+      for (int spin = 0; ld_acquire(P.bar + 1) == gen; ++spin) {
+        if ((spin & 15) != 15) continue;
         if (*(volatile int*)P.err) {
           ok = 0;
           break;
         }
-        if (gtimer() - t0 > P.timeout_ns) {
+        const unsigned long long t = gtimer();
+        if (!t0) t0 = t;
+        if (t - t0 > P.timeout_ns) {
           atomicExch(P.err, (int)LFX_TIMEOUT);
           ok = 0;
           break;
         }
-        __nanosleep(100);
       }
     }
-    __threadfence();
     if (*(volatile int*)P.err) ok = 0;
     sh.ok = ok;
   }
@@ -685,6 +686,8 @@ __device__ __noinline__ void alpha_phase(const BParams& P, BShared& sh) {
     const double* part = D->part + 2 * (int64_t)D->nch;
     const int nc = D->ncell;
     double a = 0.0;
+    // (eight loads in flight: one at a time took 11 of an iteration's 290 us)
+#pragma unroll 8
     for (int i = threadIdx.x; i < nc; i += kBT) a = a + __ldcg(part + i);
     const double pz = bsum(a, sh.red);
     if (threadIdx.x == 0) {
@@ -697,7 +700,7 @@ __device__ __noinline__ void alpha_phase(const BParams& P, BShared& sh) {
   }
 }
 
-// ---- Vector phases. An item is (slot, chunk of kBSub * RCHUNK = 16384
+// ---- Vector phases. An item is (slot, chunk of kBSub * RCHUNK = 4096
 // values). The block takes an item; each thread takes four consecutive
 // values per step (16-byte accesses, masked at the vector's end), with the
 // loads of two steps in flight before any store. The slot record is read
@@ -709,6 +712,9 @@ __device__ __noinline__ void alpha_phase(const BParams& P, BShared& sh) {
 // fixed order (lanes by butterfly, warps left to right) into the chunk's
 // partial; the last block to finish a slot's chunks (ticket) sums the
 // partials in chunk order and runs fin(record, state, totals).
+// The chunk is small so that a few slots fill the grid: twelve uneven W0 slots
+// (3.6 M rows) took 143 ms with 16384 values (220 items for 444 blocks), 139 with
+// 8192, 138 with 4096; six W2 ones 7.8, 7.6, 7.4; sixty W0 ones 469, 452, 458.
 constexpr int kVStep = kBT * 4;                   // values per block step
 constexpr int kVSteps = kBSub * RCHUNK / kVStep;  // steps per chunk (16)
 static_assert(kVSteps % 2 == 0, "two steps per pass");
