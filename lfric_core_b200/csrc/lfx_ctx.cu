@@ -111,6 +111,44 @@ int to_host_small(lfx_ctx* ctx, void* host_dev, const void* dev, size_t bytes) {
   return LFX_OK;
 }
 
+__global__ void small_copy_mark(const unsigned* __restrict__ src, unsigned* dst, int words,
+                                const int* err, int* err_dst, HostMark mark) {
+  for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+  if (threadIdx.x == 0) *err_dst = *err;
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) mark.set();
+}
+
+HostMark host_next(lfx_ctx* ctx) {
+  return HostMark{reinterpret_cast<unsigned*>(ctx->h_scalars_dev + kHostSeq), ++ctx->host_seq};
+}
+
+// The number arrives when every operation queued before its kernel is done. A
+// stream that ends without it (a failed launch) is reported.
+int host_wait(lfx_ctx* ctx) {
+  const volatile unsigned* p = reinterpret_cast<const volatile unsigned*>(ctx->h_scalars + kHostSeq);
+  for (unsigned spin = 1;; ++spin) {
+    if (*p == ctx->host_seq) return LFX_OK;
+    if (spin % 4096) continue;
+    const cudaError_t e = cudaStreamQuery(ctx->stream);
+    if (e == cudaErrorNotReady) continue;
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamQuery");
+    if (*p == ctx->host_seq) return LFX_OK;
+    return fail(ctx, LFX_CUDA_ERROR, "a result never reached the host");
+  }
+}
+
+int to_host_wait(lfx_ctx* ctx, void* host_dev, const void* dev, size_t bytes) {
+  const HostMark mark = host_next(ctx);
+  small_copy_mark<<<1, 64, 0, ctx->stream>>>((const unsigned*)dev, (unsigned*)host_dev,
+                                             (int)(bytes / 4), ctx->d_err,
+                                             reinterpret_cast<int*>(ctx->h_scalars_dev + kHostErr), mark);
+  ctx->launches++;
+  LFX_CK(ctx, cudaGetLastError());
+  return host_wait(ctx);
+}
+
 void timing_end(lfx_ctx* ctx) {
   if (!ctx->time_applies) return;
   if (ctx->capture_ev) {
@@ -153,6 +191,7 @@ int lfx_ctx_create(int device, lfx_ctx** out) {
   if (!rc)
     rc = host_alloc_mapped(ctx, (void**)&ctx->h_scalars, (void**)&ctx->h_scalars_dev,
                            sizeof(double) * 64);
+  if (!rc) std::memset(ctx->h_scalars, 0, sizeof(double) * 64);
   if (!rc) rc = ensure_partials(ctx, (int64_t)RCHUNK * 4096, 1);
   if (rc) {
     lfx_ctx_destroy(ctx);

@@ -38,6 +38,7 @@ struct lfx_ctx {
   double* d_scalars = nullptr;
   double* h_scalars = nullptr;      // pinned, mapped into the device's address space
   double* h_scalars_dev = nullptr;  // its device address
+  unsigned host_seq = 0;            // number of the last result sent to the host (see host_wait)
   int64_t device_bytes = 0;
   // operator-apply timing: event pairs, the precision of each timed apply,
   // and running totals per precision (index 0: FP64, 1: FP32)
@@ -470,6 +471,24 @@ int prec_apply_impl(lfx_prec* p, int32_t precision, const void* x, void* y, int6
 // large field copies that other streams have in flight.
 int host_alloc_mapped(lfx_ctx* ctx, void** host, void** dev, size_t bytes);
 int to_host_small(lfx_ctx* ctx, void* host_dev, const void* dev, size_t bytes);
+// A result the host waits for ends with a number (host_next) that its kernel
+// writes after it; the host looks for the number instead of synchronising the
+// stream, which returns later. h_scalars: [0, 62) results, [62] the device error
+// flag as of the last to_host_wait, [63] the number.
+constexpr int kHostErr = 62, kHostSeq = 63;
+struct HostMark {
+  unsigned* p;
+  unsigned seq;
+  __device__ void set() const {
+    if (!p) return;
+    __threadfence_system();
+    *((volatile unsigned*)p) = seq;
+  }
+};
+HostMark host_next(lfx_ctx* ctx);
+int host_wait(lfx_ctx* ctx);
+// bytes to the host with the device error flag, and waits for them
+int to_host_wait(lfx_ctx* ctx, void* host_dev, const void* dev, size_t bytes);
 void timing_begin(lfx_ctx* ctx, int32_t precision);
 void timing_end(lfx_ctx* ctx);
 }  // namespace lfx

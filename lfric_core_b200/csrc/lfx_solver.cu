@@ -96,10 +96,7 @@ size_t gm_doubles(int K) { return 2 * (size_t)(K + 1) * K + 2 * (size_t)(K + 1) 
 
 int read_state(lfx_solver* s) {
   lfx_ctx* ctx = s->ctx;
-  int rc = to_host_small(ctx, s->h_state_dev, s->d_state, sizeof(DevState));
-  if (rc) return rc;
-  LFX_CK(ctx, cudaStreamSynchronize(ctx->stream));
-  return LFX_OK;
+  return to_host_wait(ctx, s->h_state_dev, s->d_state, sizeof(DevState));
 }
 
 // the initial state travels as a kernel argument (no copy engine involved)
@@ -1417,9 +1414,8 @@ int refined_run(lfx_solver* s, lfx_vec* xv, const lfx_vec* bv, lfx_solve_info* i
     int q = op_apply_impl(s->op, x, r, b, nullptr);
     if (q) return q;
     q = norm_kernel(ctx, n, (const double*)r, sc, nullptr);
-    if (!q) q = to_host_small(ctx, ctx->h_scalars_dev, sc, 8);
+    if (!q) q = to_host_wait(ctx, ctx->h_scalars_dev, sc, 8);
     if (q) return q;
-    LFX_CK(ctx, cudaStreamSynchronize(ctx->stream));
     *out = ctx->h_scalars[0];
     return LFX_OK;
   };
@@ -1432,9 +1428,8 @@ int refined_run(lfx_solver* s, lfx_vec* xv, const lfx_vec* bv, lfx_solve_info* i
     // the first residual skips its apply when x starts at zero
     int q = residual_from<double>(s, s->op, x, r, b, &s->d_state->x_zero);
     if (!q) q = norm_kernel(ctx, n, (const double*)r, sc, nullptr);
-    if (!q) q = to_host_small(ctx, ctx->h_scalars_dev, sc, 8);
+    if (!q) q = to_host_wait(ctx, ctx->h_scalars_dev, sc, 8);
     if (q) return q;
-    LFX_CK(ctx, cudaStreamSynchronize(ctx->stream));
     r0 = ctx->h_scalars[0];
   }
   memset(info, 0, sizeof *info);
@@ -1661,7 +1656,9 @@ int lfx_solver_apply(lfx_solver* s, lfx_vec* x, const lfx_vec* b, lfx_solve_info
     if (!rc) fill_info(s, info);  // (each of them ends with the state read)
   }
   if (ctx->time_applies) drain_timing(ctx);
-  if (!rc) rc = lfx_ctx_check_device_error(ctx);
+  // (the device error flag came with the last state or norm)
+  if (!rc && *reinterpret_cast<const volatile int*>(ctx->h_scalars + kHostErr))
+    rc = lfx_ctx_check_device_error(ctx);
   if (rc) {
     info->status = rc;
     return rc;

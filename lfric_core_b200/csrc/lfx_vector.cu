@@ -53,13 +53,16 @@ static int k_scale(lfx_ctx* ctx, T* x, T a, int64_t n) {
       [=] __device__(int64_t i, const V1<T>& v, double*) { x[i] = a * v.a; }, NoFin{});
 }
 template <class T>
-static int k_dot(lfx_ctx* ctx, const T* x, const T* y, int64_t n, double* out) {
+static int k_dot(lfx_ctx* ctx, const T* x, const T* y, int64_t n, double* out, HostMark mark) {
   return launch_chunks<1>(
       ctx, n, [=] __device__(int64_t i) { return V2<T>{x[i], y[i]}; },
       [=] __device__(int64_t, const V2<T>& v, double* acc) {
         acc[0] = fma((double)v.a, (double)v.b, acc[0]);
       },
-      [=] __device__(const double* tot) { *out = tot[0]; });
+      [=] __device__(const double* tot) {
+        *out = tot[0];
+        mark.set();
+      });
 }
 template <class S, class D>
 static int k_convert(lfx_ctx* ctx, D* d, const S* s, int64_t n) {
@@ -81,11 +84,13 @@ static bool same_shape(const lfx_vec* a, const lfx_vec* b) {
   return fail((a)->ctx, LFX_TYPE_MISMATCH, "vectors differ in shape or precision")
 
 // result of NF per-field sums combined left to right on the host, as the
-// field loops of sci_field_vector_mod.x90:132-182 do
+// field loops of sci_field_vector_mod.x90:132-182 do. The reductions write their
+// sums to the mapped h_scalars themselves and the last one marks the end: a dot
+// of 210 816 values by a copy kernel and a stream synchronisation after it took
+// 14 us as the caller sees it.
 static int read_sums(lfx_ctx* ctx, int nf, double* out_sum) {
-  int rc = to_host_small(ctx, ctx->h_scalars_dev, ctx->d_scalars, sizeof(double) * nf);
+  const int rc = host_wait(ctx);
   if (rc) return rc;
-  LFX_CK(ctx, cudaStreamSynchronize(ctx->stream));
   double s = 0.0;
   for (int f = 0; f < nf; ++f) s = s + ctx->h_scalars[f];
   *out_sum = s;
@@ -218,11 +223,13 @@ int lfx_vec_dot(const lfx_vec* v, const lfx_vec* x, double* out) {
   lfx_ctx* ctx = v->ctx;
   int nf = (int)v->data.size();
   for (int f = 0; f < nf; ++f) {
+    const HostMark mark = f == nf - 1 ? host_next(ctx) : HostMark{nullptr, 0u};
+    double* sum = ctx->h_scalars_dev + f;
     int rc = v->precision == LFX_R64
-                 ? k_dot(ctx, (const double*)v->data[f], (const double*)x->data[f], v->undf[f],
-                         ctx->d_scalars + f)
-                 : k_dot(ctx, (const float*)v->data[f], (const float*)x->data[f], v->undf[f],
-                         ctx->d_scalars + f);
+                 ? k_dot(ctx, (const double*)v->data[f], (const double*)x->data[f], v->undf[f], sum,
+                         mark)
+                 : k_dot(ctx, (const float*)v->data[f], (const float*)x->data[f], v->undf[f], sum,
+                         mark);
     if (rc) return rc;
   }
   return read_sums(ctx, nf, out);
@@ -242,11 +249,12 @@ int lfx_vec_field_norm(const lfx_vec* v, int32_t position, double* out) {
     return fail(v->ctx, LFX_INVALID_ARGUMENT, "field position out of range");
   lfx_ctx* ctx = v->ctx;
   int f = position - 1;
+  const HostMark mark = host_next(ctx);
   int rc = v->precision == LFX_R64
                ? k_dot(ctx, (const double*)v->data[f], (const double*)v->data[f], v->undf[f],
-                       ctx->d_scalars)
+                       ctx->h_scalars_dev, mark)
                : k_dot(ctx, (const float*)v->data[f], (const float*)v->data[f], v->undf[f],
-                       ctx->d_scalars);
+                       ctx->h_scalars_dev, mark);
   if (rc) return rc;
   double s;
   rc = read_sums(ctx, 1, &s);
