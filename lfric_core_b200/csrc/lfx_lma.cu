@@ -1642,27 +1642,6 @@ int build_layout(lfx_ctx* ctx, lfx_lma_layout* L, int32_t ncell, int32_t nl, int
       L->cs_struct_part = cs_part[0];
     }
   }
-  if (!mf0) {
-    // descriptors of the transpose apply on faces, where every column has at
-    // most two records (the to-space dof is filled in by the caller)
-    std::vector<int4> d((size_t)L->nent * 3, make_int4(0, 0, 0, 0));
-    bool ok = true;
-    for (int32_t e = 0; ok && e < L->nent; ++e) {
-      int n = 0;
-      for (int32_t g = ent_grp[e]; g < ent_grp[e + 1]; ++g)
-        for (int o = max_off; o >= 0; --o)
-          for (int r = 0; r < rec_n(grp_rec[g]); ++r) {
-            if (rec_off(grp_rec[g], r) != o) continue;
-            if (n < 2)
-              d[3 * (size_t)e + 1 + n] =
-                  make_int4(grp_cell[g], rec_df(grp_rec[g], r) * nl, o, 0);
-            ++n;
-          }
-      ok = n <= 2;
-      d[3 * (size_t)e] = make_int4(ent_base[e], ent_h[e], n, 0);
-    }
-    if (ok) up((void**)&L->tdesc, d.data(), d.size() * sizeof(int4));
-  }
   if (mf0) {
     std::vector<int4> ep(L->nent);
     for (int32_t e = 0; e < L->nent; ++e) ep[e] = make_int4(ent_base[e], ent_h[e], ent_grp[e], ent_grp[e + 1]);
@@ -2428,11 +2407,33 @@ int x_plus_ay_copy(lfx_ctx* ctx, int32_t precision, const void* x, double a, con
   return LFX_OK;
 }
 
-// the first to-space dof of each descriptor's cells
-static __global__ void tdesc_map(int nent, int ndf_to, const int32_t* __restrict__ map_to, int4* td) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * nent || i % 3 == 0) return;
-  td[i].w = map_to[(size_t)td[i].x * ndf_to];
+// descriptors of lma_faces_t (columns of at most two records)
+static __global__ void tdesc_build(LayoutArgs A, int max_off, int ndf_to,
+                                   const int32_t* __restrict__ map_to, int4* td) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= A.nent) return;
+  int n = 0;
+  for (int g = A.ent_grp[e]; g < A.ent_grp[e + 1]; ++g) {
+    const uint32_t pk = A.grp_rec[g];
+    const int c = A.grp_cell[g];
+    for (int o = max_off; o >= 0; --o)
+      for (int r = 0; r < rec_n(pk); ++r) {
+        if (rec_off(pk, r) != o || n == 2) continue;
+        td[3 * (size_t)e + 1 + n++] =
+            make_int4(c, rec_df(pk, r) * A.nlayers, o, map_to[(size_t)c * ndf_to]);
+      }
+  }
+  for (int q = n; q < 2; ++q) td[3 * (size_t)e + 1 + q] = make_int4(0, 0, 0, 0);
+  td[3 * (size_t)e] = make_int4(A.ent_base[e], A.ent_h[e], n, 0);
+}
+
+static int make_tdesc(lfx_ctx* ctx, const lfx_lma_layout* L, lfx_lma_layout* T) {
+  const int rc = dmalloc(ctx, (void**)&T->tdesc, (size_t)T->nent * 48);
+  if (rc) return rc;
+  tdesc_build<<<(T->nent + 255) / 256, 256, 0, ctx->stream>>>(args_of(T, 0), T->max_off, L->ndf_to,
+                                                              L->map_to, T->tdesc);
+  LFX_CK(ctx, cudaGetLastError());
+  return LFX_OK;
 }
 
 // one resident wave of blocks
@@ -2822,9 +2823,9 @@ int lfx_op_apply_transpose(lfx_op* op, const lfx_vec* x, lfx_vec* y) {
       return rc;
     }
     L->tlay = T;
-    if (T->tdesc)
-      tdesc_map<<<(3 * T->nent + 255) / 256, 256, 0, ctx->stream>>>(T->nent, L->ndf_to, L->map_to,
-                                                                    T->tdesc);
+    if (T->nent && T->max_blocks <= 2 && (L->ndf_to == 1 || L->ndf_to == 6) &&
+        (rc = make_tdesc(ctx, L, T)))
+      return rc;
   }
   lfx_lma_layout* T = L->tlay;
   if (!T->full_cover)

@@ -7,7 +7,7 @@
 // last block of the fused reduction kernel that produces it (see
 // chunk_kernel), so an iteration issues no host round trip. Kernels take a
 // "done" flag and return at once when it is set. The kernel sequence of one
-// GMRES restart cycle, or of 8 CG / BiCGStab iterations, is captured once into
+// GMRES restart cycle, of 8 CG or 4 BiCGStab iterations, is captured once into
 // a CUDA graph (per solution / right-hand-side buffer pair) and replayed; the
 // host reads the flag once per replay. Vector updates that the reference
 // performs as separate builtins are fused when the fusion does not change a
@@ -797,6 +797,10 @@ int cg_run(lfx_solver* s, T* x, const T* b) {
 }
 
 // ------------------------------------------------------------------ BiCGStab
+// iterations of one graph: a solve ends with up to three idle ones (17 launches
+// each) and captures them for every new pair of vectors. With eight the C37 x 23
+// W2 solve (12 iterations) took 1167 us, its first pass 1853.
+constexpr int kBicgIters = 4;
 template <class T>
 int bicgstab_run(lfx_solver* s, T* x, const T* b) {
   lfx_ctx* ctx = s->ctx;
@@ -834,7 +838,7 @@ int bicgstab_run(lfx_solver* s, T* x, const T* b) {
   if (rc) return rc;
   auto batch = [&]() -> int {
     int q;
-    for (int it = 0; it < 8; ++it) {
+    for (int it = 0; it < kBicgIters; ++it) {
       // rho = <r, r0> ; beta = (rho/rho_old)(alpha/omega)
       q = launch_chunks<1>(
           ctx, n, [=] __device__(int64_t i) { return V2<T>{r[i], r0[i]}; },
