@@ -1522,19 +1522,16 @@ int lfx_mrhs_create(const lfx_op* op, int32_t kind, int32_t nrhs, int32_t cells_
   m->max_colours = max_col;
   m->nent = nent;
   int rc = LFX_OK;
-  // the columns each column couples to: those sharing a cell, by first dof,
-  // then the column itself; and the cells around it
+  // the columns each column couples to: those sharing a cell, in the order they
+  // are met, then the column itself; and the cells around it
   std::vector<int> h_base, h_off{0}, h_nbr, h_coff{0};
   std::vector<int4> h_ccell;
-  std::vector<int32_t> near;
+  h_nbr.reserve((size_t)nv * 9);
+  h_ccell.reserve(vcells.size());
+  int32_t near[kMaxSlot];
   for (int id : h_own) {
-    near.clear();
-    for (int k = voff[id]; k < voff[id + 1]; ++k)
-      for (int v = 0; v < 4; ++v) near.push_back(vbase[cv[(size_t)vcells[k] * 4 + v]]);
-    std::sort(near.begin(), near.end());
-    near.erase(std::unique(near.begin(), near.end()), near.end());
-    near.erase(std::find(near.begin(), near.end(), vbase[id]));
-    near.push_back(vbase[id]);
+    int nn = 0;
+    const size_t e0 = h_ccell.size();
     for (int k = voff[id]; k < voff[id + 1]; ++k) {
       const int c = vcells[k];
       // (a cell that holds the column at two of its vertices is listed once
@@ -1544,19 +1541,33 @@ int lfx_mrhs_create(const lfx_op* op, int32_t kind, int32_t nrhs, int32_t cells_
       unsigned slots = 0u;
       int mine = -1;
       for (int v = 0; v < 4; ++v) {
-        const int32_t u = vbase[cv[(size_t)c * 4 + v]];
-        const auto it = u == vbase[id] ? near.end() - 1 : std::find(near.begin(), near.end() - 1, u);
-        slots |= (unsigned)(it - near.begin()) << (8 * v);
-        if (u == vbase[id] && seen-- == 0) mine = v;
+        const int32_t u = cv[(size_t)c * 4 + v];
+        int t = 255;  // the column itself: its slot is known at the end
+        if (u != id) {
+          for (t = 0; t < nn && near[t] != u; ++t) {
+          }
+          if (t == kMaxSlot - 1) {
+            rc = fail(ctx, LFX_NOT_SUPPORTED, "a vertex column has too many neighbours");
+            t = 0;
+          } else if (t == nn) {
+            near[nn++] = u;
+          }
+        } else if (seen-- == 0) {
+          mine = v;
+        }
+        slots |= (unsigned)t << (8 * v);
       }
       h_ccell.push_back(make_int4(c, mine, (int)slots, 0));
     }
+    for (size_t e = e0; e < h_ccell.size(); ++e)
+      for (int v = 0; v < 4; ++v)
+        if ((((unsigned)h_ccell[e].z >> (8 * v)) & 255u) == 255u)
+          h_ccell[e].z = (int)(((unsigned)h_ccell[e].z & ~(255u << (8 * v))) | ((unsigned)nn << (8 * v)));
     h_base.push_back(vbase[id]);
-    h_nbr.insert(h_nbr.end(), near.begin(), near.end());
+    for (int t = 0; t < nn; ++t) h_nbr.push_back(vbase[near[t]]);
+    h_nbr.push_back(vbase[id]);
     h_off.push_back((int)h_nbr.size());
     h_coff.push_back((int)h_ccell.size());
-    if (near.size() > (size_t)kMaxSlot)
-      rc = fail(ctx, LFX_NOT_SUPPORTED, "a vertex column has too many neighbours");
   }
   auto up = [&](void** dst, size_t* held, const void* src, size_t bytes) {
     if (rc) return;
