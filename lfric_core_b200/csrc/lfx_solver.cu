@@ -628,14 +628,42 @@ int cg_persist_launch(lfx_ctx* ctx, CgArgs<T> A, DevState* S, const DevState& in
   return LFX_OK;
 }
 
+// whether the device holds a cluster of kCgCluster such blocks
+template <class T, int N, bool EDGE>
+bool cg_cluster_fits(const lfx_ctx* ctx) {
+  static int fits = -1;
+  if (fits < 0) {
+    auto kern = cg_persist<T, N, true, EDGE, DevState>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgSmemMax);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kCgCluster);
+    cfg.blockDim = dim3(kCgThreads);
+    cfg.dynamicSmemBytes = kCgSmemMax;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kCgCluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    fits = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
+    cudaGetLastError();
+  }
+  return fits == 1;
+}
+
 template <class T, int N>
 int cg_persist_form(lfx_ctx* ctx, const CgArgs<T>& A, DevState* S, const DevState& init, int first,
                     const CgShape& q) {
   if (q.edge)
-    return q.cluster ? cg_persist_launch<T, N, true, true>(ctx, A, S, init, first, q.grid)
-                     : cg_persist_launch<T, N, false, true>(ctx, A, S, init, first, q.grid);
-  return q.cluster ? cg_persist_launch<T, N, true, false>(ctx, A, S, init, first, q.grid)
-                   : cg_persist_launch<T, N, false, false>(ctx, A, S, init, first, q.grid);
+    return q.cluster && cg_cluster_fits<T, N, true>(ctx)
+               ? cg_persist_launch<T, N, true, true>(ctx, A, S, init, first, q.grid)
+               : cg_persist_launch<T, N, false, true>(ctx, A, S, init, first, q.grid);
+  return q.cluster && cg_cluster_fits<T, N, false>(ctx)
+             ? cg_persist_launch<T, N, true, false>(ctx, A, S, init, first, q.grid)
+             : cg_persist_launch<T, N, false, false>(ctx, A, S, init, first, q.grid);
 }
 
 // the whole solve
