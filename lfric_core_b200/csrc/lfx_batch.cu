@@ -35,7 +35,7 @@
 //   P   p = z + beta p
 // Work items: apply items of up to `cells_per_item` cell columns of one
 // colour of one slot, one warp each (a column's segments in order);
-// 4096-value chunk items (slot, chunk), one block each, for the vector
+// 4096-value chunk items (slot, one chunk or four), one block each, for the vector
 // phases; 64-column items for the sweeps. Per-slot sums are reduced in an
 // order fixed by the slot alone (per cell column, per 4096-value chunk, then
 // in index order), so a slot's result is bit-identical whatever else is in
@@ -66,6 +66,7 @@ constexpr int kBT = 256;         // threads per block of the persistent kernel
 constexpr int kBW = kBT / 32;    // warps per block
 constexpr int kMaxBps = 3;       // blocks per SM the kernel is built for (launch bounds)
 constexpr int kBSub = 2;         // a chunk item: kBSub chunks of RCHUNK values (4096)
+constexpr int kChGroup = 4;       // chunks a chunk item covers when there are many
 constexpr int kMaxIters = 64;    // super-iterations per launch, at most
 constexpr int kMaxSeg = 4;       // warps (segments of <= 31 levels) per cell column, at most
 constexpr int kMaxColours = 8;   // cell colours of a slot, at most
@@ -132,7 +133,7 @@ struct BParams {
   const int* off32;     // [ncolour * ngr32 + 1]: items of group g, colour c from off32[g ncolour + c]
   const int4* items64;  // FP64 residual items {slot, q0, columns, 0}
   const int* off64;
-  const int2* chunks;   // {slot, chunk}
+  const int2* chunks;   // {slot, group of chgrp chunks}
   const int2* cols;     // {slot, column}
   const int* slotlist;  // the slots the lists cover
   const BSlot* slots;
@@ -144,14 +145,14 @@ struct BParams {
   int* err;             // LFX_TIMEOUT when a wait ran out
   int ngr32, ngr64, nchunk, ncolitem;
   int iters, max_slots, any_cma, ncolour;
-  int nslot, pad1;
+  int nslot, chgrp;
   unsigned long long timeout_ns;
 };
 
 struct BShared {
   int last;
   double red[kBT / 32];
-  double red2[2][kBT / 32];
+  double red2[kChGroup][2][kBT / 32];
   int ok;
 };
 
@@ -700,8 +701,8 @@ __device__ __noinline__ void alpha_phase(const BParams& P, BShared& sh) {
   }
 }
 
-// ---- Vector phases. An item is (slot, chunk of kBSub * RCHUNK = 4096
-// values). The block takes an item; each thread takes four consecutive
+// ---- Vector phases. An item is (slot, chunks of kBSub * RCHUNK = 4096
+// values: one, or kChGroup of them). The block takes an item; each thread takes four consecutive
 // values per step (16-byte accesses, masked at the vector's end), with the
 // loads of two steps in flight before any store. The slot record is read
 // where it lies (read-only during a launch: broadcast loads); the state
@@ -715,6 +716,11 @@ __device__ __noinline__ void alpha_phase(const BParams& P, BShared& sh) {
 // The chunk is small so that a few slots fill the grid: twelve uneven W0 slots
 // (3.6 M rows) took 143 ms with 16384 values (220 items for 444 blocks), 139 with
 // 8192, 138 with 4096; six W2 ones 7.8, 7.6, 7.4; sixty W0 ones 469, 452, 458.
+// Where that gives every block of the largest grid 4 kChGroup chunks or more, an item
+// takes kChGroup of them (each with its own partial, so the bits stay), with one
+// block sum and one ticket an item: 256 uneven W0 slots (63 M rows, 15 424 chunks)
+// took 3388 us an iteration with a chunk an item, 3291 so (3240-3270 with chunks of
+// 16384 values, which cost the few slots above).
 constexpr int kVStep = kBT * 4;                   // values per block step
 constexpr int kVSteps = kBSub * RCHUNK / kVStep;  // steps per chunk (16)
 static_assert(kVSteps % 2 == 0, "two steps per pass");
@@ -790,7 +796,7 @@ __device__ __noinline__ void vec_phase(const BParams& P, BShared& sh, Pred pred,
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int u = blockIdx.x; u < P.nchunk; u += gridDim.x) {
     const int2 item = __ldg(P.chunks + u);
-    const int s = item.x, ch = item.y;
+    const int s = item.x;
     const BState* Sg = P.st + s;
     if (!pred(__ldcg(&Sg->phase), __ldcg(&Sg->flag))) continue;  // block-uniform
     const BSlot& D = P.slots[s];
@@ -800,37 +806,46 @@ __device__ __noinline__ void vec_phase(const BParams& P, BShared& sh, Pred pred,
     V.alpha = (float)__ldcg(&Sg->alpha);
     V.beta = (float)__ldcg(&Sg->beta);
     const int64_t n = D.n;
-    double acc[NR > 0 ? NR : 1];
+    const int ch0 = item.y * P.chgrp, nk = min(P.chgrp, D.nch - ch0);
+    for (int k = 0; k < nk; ++k) {
+      double acc[NR > 0 ? NR : 1];
 #pragma unroll
-    for (int r = 0; r < (NR > 0 ? NR : 1); ++r) acc[r] = 0.0;
-    const int64_t c0 = (int64_t)ch * (kBSub * RCHUNK);
-    for (int stp = 0; stp < kVSteps; stp += 2) {
-      if (c0 + (int64_t)stp * kVStep >= n) break;  // block-uniform
-      const int64_t i0 = c0 + (int64_t)stp * kVStep + 4 * threadIdx.x, i1 = i0 + kVStep;
-      const auto a = ld(D, i0, n);
-      const auto b = ld(D, i1, n);
-      if (i0 < n) op(D, V, i0, n, a, acc);
-      if (i1 < n) op(D, V, i1, n, b, acc);
+      for (int r = 0; r < (NR > 0 ? NR : 1); ++r) acc[r] = 0.0;
+      const int64_t c0 = (int64_t)(ch0 + k) * (kBSub * RCHUNK);
+      for (int stp = 0; stp < kVSteps; stp += 2) {
+        if (c0 + (int64_t)stp * kVStep >= n) break;  // block-uniform
+        const int64_t i0 = c0 + (int64_t)stp * kVStep + 4 * threadIdx.x, i1 = i0 + kVStep;
+        const auto a = ld(D, i0, n);
+        const auto b = ld(D, i1, n);
+        if (i0 < n) op(D, V, i0, n, a, acc);
+        if (i1 < n) op(D, V, i1, n, b, acc);
+      }
+      if constexpr (NR > 0) {
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          const double t = warp_butterfly(acc[r]);
+          if (lane == 0) sh.red2[k][r][w] = t;
+        }
+      }
     }
     if constexpr (NR > 0) {
       const int nch = D.nch;
       double* part = D.part;
-#pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        const double t = warp_butterfly(acc[r]);
-        if (lane == 0) sh.red2[r][w] = t;
-      }
       __syncthreads();
-      if (threadIdx.x == 0) {
+      if (w == 0) {
+        if (lane < nk * NR) {
+          const int k = lane / NR, r = lane % NR;
+          double t = sh.red2[k][r][0];
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          double t = sh.red2[r][0];
-#pragma unroll
-          for (int q = 1; q < kBW; ++q) t = t + sh.red2[r][q];
-          __stcg(part + (int64_t)r * nch + ch, t);
+          for (int q = 1; q < kBW; ++q) t = t + sh.red2[k][r][q];
+          __stcg(part + (int64_t)r * nch + ch0 + k, t);
+          __threadfence();
         }
-        __threadfence();
-        sh.last = atomicAdd(&P.tickets[s], 1u) == (unsigned)nch - 1u;
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence();
+          sh.last = atomicAdd(&P.tickets[s], (unsigned)nk) == (unsigned)(nch - nk);
+        }
       }
       __syncthreads();
       if (sh.last) {
@@ -841,16 +856,16 @@ __device__ __noinline__ void vec_phase(const BParams& P, BShared& sh, Pred pred,
           a[r] = 0.0;
           for (int i = threadIdx.x; i < nch; i += kBT) a[r] = a[r] + __ldcg(part + (int64_t)r * nch + i);
           const double t = warp_butterfly(a[r]);
-          if (lane == 0) sh.red2[r][w] = t;
+          if (lane == 0) sh.red2[0][r][w] = t;
         }
         __syncthreads();
         if (threadIdx.x == 0) {
           double tot[NR];
 #pragma unroll
           for (int r = 0; r < NR; ++r) {
-            tot[r] = sh.red2[r][0];
+            tot[r] = sh.red2[0][r][0];
 #pragma unroll
-            for (int q = 1; q < kBW; ++q) tot[r] = tot[r] + sh.red2[r][q];
+            for (int q = 1; q < kBW; ++q) tot[r] = tot[r] + sh.red2[0][r][q];
           }
           BState S;
           copy_state_in(&S, P.st + s);
@@ -1430,10 +1445,14 @@ int rebuild(lfx_batch* B) {
   const int64_t n32 = build_apply_runs(B, act, ncolour, 8, r32, off32);
   const int64_t n64 = build_apply_runs(B, act, ncolour, 16, r64, off64);
   int64_t nch = 0, ncol = 0;
+  for (int s : act) nch += B->slots[s].nch;
+  // (vec_phase says why)
+  const int chgrp = nch >= (int64_t)kChGroup * 4 * kMaxBps * ctx->num_sms ? kChGroup : 1;
+  nch = 0;
   for (int s : act) {
     const SlotHost& H = B->slots[s];
-    rch.push_back(ListRun{s, 0, H.nch, (int)nch});
-    nch += H.nch;
+    rch.push_back(ListRun{s, 0, (H.nch + chgrp - 1) / chgrp, (int)nch});
+    nch += (H.nch + chgrp - 1) / chgrp;
     if (H.cma && H.ncol > 0) {
       rcol.push_back(ListRun{s, 0, H.ncol, (int)ncol});
       ncol += H.ncol;
@@ -1507,6 +1526,7 @@ int rebuild(lfx_batch* B) {
   P.ngr64 = (int)(off64.size() - 1) / ncolour;
   P.ncolour = ncolour;
   P.nchunk = (int)nch;
+  P.chgrp = chgrp;
   P.ncolitem = (int)ncol;
   P.iters = B->iters;
   P.max_slots = B->max_slots;
