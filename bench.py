@@ -20,8 +20,8 @@ tridiagonal on the vertical faces and Jacobi on the horizontal faces.
             headline pass runs without them)
   cpu_baseline  the oracle (CPU restatement of the reference) on this host
   workloads the other configurations: plain FP64 CG on C24x20 W0 against the
-            oracle; 64 right-hand sides of C48x30 W0 with tensor-core (TF32 /
-            BF16) applies in FP64 refinement; 256 batched uneven W0 solves;
+            oracle; 64 right-hand sides of C48x30 W0 with FP32 column-stencil
+            applies in FP64 refinement; 256 batched uneven W0 solves;
             a Poisson stream of W2 requests served by continuous batching
 
 --impl reference times the oracle port on the host cores instead (the
@@ -335,9 +335,8 @@ def leg_plain_cg(ctx, lfx, mg, wl, torch, stream, nsolves=50, ncpu=5):
 
 def leg_multi_rhs(ctx, lfx, mg, wl, torch, stream, n=48, nl=30, nrhs=64):
     """64 seeded N(0,1) right-hand sides of the C48x30 W0 mass+diffusion
-    operator solved together: FP64 refinement around an FP32 Jacobi CG whose
-    per-cell products run as (64 x 8).(8 x 8) tensor-core GEMMs in TF32 and in
-    BF16, against 64 serial plain FP64 device CG solves; per-RHS error of the
+    operator solved together: FP64 refinement around an FP32 Jacobi CG on column
+    stencils (both kinds of operator), against 64 serial plain FP64 device CG solves; per-RHS error of the
     solution against the FP64 solve."""
     p = mg.w0_problem(n, nl, seed=1, rhs="normal")
     s = wl.device_w0(ctx, p)
@@ -363,7 +362,7 @@ def leg_multi_rhs(ctx, lfx, mg, wl, torch, stream, n=48, nl=30, nrhs=64):
     ctx.synchronize()
     t64 = ev[0].elapsed_time(ev[1]) / 1e3
     out = {"workload": f"C{n}x{nl} W0 mass+diffusion, {nrhs} N(0,1) right-hand sides, 1e-8 rel. "
-                       "residual, Jacobi; FP32 CG with tensor-core apply inside FP64 refinement",
+                       "residual, Jacobi; FP32 CG with column-stencil apply inside FP64 refinement",
            "undf": p.undf, "ncell_3d": p.mesh.ncell_3d,
            "serial_fp64_solves_per_s": round(nrhs / t64, 2), "serial_fp64_s": round(t64, 4),
            "serial_fp64_iterations_max": max(it64)}
