@@ -722,7 +722,7 @@ __device__ __noinline__ void alpha_phase(const BParams& P, BShared& sh) {
 // took 3388 us an iteration with a chunk an item, 3291 so (3240-3270 with chunks of
 // 16384 values, which cost the few slots above).
 constexpr int kVStep = kBT * 4;                   // values per block step
-constexpr int kVSteps = kBSub * RCHUNK / kVStep;  // steps per chunk (16)
+constexpr int kVSteps = kBSub * RCHUNK / kVStep;  // steps per chunk (4)
 static_assert(kVSteps % 2 == 0, "two steps per pass");
 
 struct VState {
