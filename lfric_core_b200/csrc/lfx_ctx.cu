@@ -38,6 +38,9 @@ void dfree(lfx_ctx* ctx, void* p, size_t bytes) {
   ctx->device_bytes -= (int64_t)bytes;
 }
 
+// An outgrown buffer stays until the context goes: graphs that solvers have
+// captured write through its address. (Each is less than half the next one's
+// size, so all of them together are smaller than the buffer in use.)
 int ensure_partials(lfx_ctx* ctx, int64_t n, int nsums) {
   int64_t need = nchunks(n) * nsums;
   if (need < 1) need = 1;
@@ -47,13 +50,12 @@ int ensure_partials(lfx_ctx* ctx, int64_t n, int nsums) {
   cudaStreamIsCapturing(ctx->stream, &cs);
   if (cs != cudaStreamCaptureStatusNone)
     return fail(ctx, LFX_INVALID_ARGUMENT, "reduction scratch too small inside a capture");
-  LFX_CK(ctx, cudaStreamSynchronize(ctx->stream));
-  dfree(ctx, ctx->d_partials, sizeof(double) * ctx->partials_cap);
-  ctx->d_partials = nullptr;
-  ctx->partials_cap = 0;
-  int64_t cap = need * 2;
-  int rc = dmalloc(ctx, (void**)&ctx->d_partials, sizeof(double) * cap);
+  const int64_t cap = need * 2;
+  double* p = nullptr;
+  int rc = dmalloc(ctx, (void**)&p, sizeof(double) * cap);
   if (rc) return rc;
+  if (ctx->d_partials) ctx->old_partials.emplace_back(ctx->d_partials, ctx->partials_cap);
+  ctx->d_partials = p;
   ctx->partials_cap = cap;
   return LFX_OK;
 }
@@ -207,6 +209,7 @@ int lfx_ctx_destroy(lfx_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   for (auto e : ctx->ev_pool) cudaEventDestroy(e);
   dfree(ctx, ctx->d_partials, sizeof(double) * ctx->partials_cap);
+  for (auto& o : ctx->old_partials) dfree(ctx, o.first, sizeof(double) * o.second);
   dfree(ctx, ctx->d_ticket, sizeof(unsigned) * 4);
   dfree(ctx, ctx->d_scalars, sizeof(double) * 64);
   dfree(ctx, ctx->d_err, sizeof(int) * 4);

@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "lfx.h"
@@ -33,6 +34,7 @@ struct lfx_ctx {
   // reduction scratch: partials of up to 4 simultaneous sums, one ticket
   double* d_partials = nullptr;
   int64_t partials_cap = 0;  // doubles
+  std::vector<std::pair<double*, int64_t>> old_partials;  // outgrown ones (see ensure_partials)
   unsigned* d_ticket = nullptr;  // [0] of the reductions, [1..2] barrier of the persistent solver launches
   // small device scratch for scalar results of the C-ABI reductions
   double* d_scalars = nullptr;
