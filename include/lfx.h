@@ -390,6 +390,10 @@ int lfx_ctx_set_apply_kernel(lfx_ctx* ctx, int32_t which);
 /* LFX_TIMEOUT if a kernel's bounded device-side wait ran out since the last
  * check (the kernel then skipped its work); synchronises the stream */
 int lfx_ctx_check_device_error(lfx_ctx* ctx);
+/* longest wait (0 to 60 s, 2 s at first) at a barrier of the persistent CG and
+ * GMRES launches; past it the solve returns LFX_TIMEOUT and the context stays
+ * usable. A GMRES keeps the limit it had when it first met a pair of vectors. */
+int lfx_ctx_set_wait_limit(lfx_ctx* ctx, double seconds);
 
 /* ------------------------------------------------------------------ batched solves
  * Continuous batching of many independent SPD solves (no counterpart in the

@@ -30,6 +30,18 @@ constexpr size_t kCgSmemMax = 224 * 1024;
 // iterations of one launch (the next one carries on from the device state)
 constexpr int kCgItersPerLaunch = 2000;
 
+// barrier of a launch whose blocks are all resident
+struct GridBar {
+  unsigned* words;  // {arrivals, blocks gone}, zero between launches
+  int* err;         // the context's error flag
+  unsigned long long limit_ns;  // longest wait
+  int poll;         // the clock and the flag are looked at every poll + 1 polls
+};
+inline GridBar grid_bar(const lfx_ctx* ctx) {
+  // (a look costs more than a poll; a limit below a barrier's own time looks at once)
+  return GridBar{ctx->d_ticket + 1, ctx->d_err, ctx->wait_ns, ctx->wait_ns < 1000000ull ? 0 : 255};
+}
+
 template <class T>
 struct CgArgs {
   // gather layout of the operator and its matrix (lfx_lma_layout, lfx_op)
@@ -43,8 +55,7 @@ struct CgArgs {
   T *x, *r, *p, *z;
   const T* dg;
   double* partials;  // 3 nch
-  unsigned* bar;     // {arrivals, blocks gone}, zero between launches
-  int* err;
+  GridBar bar;
   int iters;
   const T* b;
   // shared memory: the vectors of the block's chunks, then as many of its dof
@@ -70,11 +81,20 @@ __device__ __forceinline__ unsigned long long cg_clock() {
   return t;
 }
 
+// A launch that comes after a wait ran out (the host has not looked yet) leaves
+// at once: the barrier's words are not zero. The whole block decides alike.
+__device__ __forceinline__ bool grid_error(const GridBar& B) {
+  return *((volatile const int*)B.err) != 0;
+}
+__device__ __forceinline__ bool grid_failed(const GridBar& B) {
+  return __syncthreads_or(grid_error(B)) != 0;
+}
+
 // All blocks of the grid (every one resident: a cooperative launch, or one
-// cluster). The grid form counts arrivals up; a wait of more than 2 s sets
+// cluster). The grid form counts arrivals up; a wait past the limit sets
 // LFX_TIMEOUT and every block leaves.
 template <bool CLUSTER>
-__device__ __forceinline__ bool cg_barrier(unsigned* bar, int* err, unsigned& target, int* ok) {
+__device__ __forceinline__ bool cg_barrier(const GridBar& B, unsigned& target, int* ok) {
   if constexpr (CLUSTER) {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
                      : "memory");
@@ -83,18 +103,18 @@ __device__ __forceinline__ bool cg_barrier(unsigned* bar, int* err, unsigned& ta
     target += gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0) {
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(B.words) : "memory");
       *ok = 1;
       unsigned long long t0 = 0;
       for (int spin = 0;; ++spin) {
         unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(B.words) : "memory");
         if ((int)(v - target) >= 0) break;
-        if ((spin & 255) == 255) {
+        if ((spin & B.poll) == B.poll) {
           const unsigned long long t = cg_clock();
           if (!t0) t0 = t;
-          if (*((volatile int*)err) || t - t0 > 2000000000ull) {
-            atomicExch(err, 1);
+          if (grid_error(B) || t - t0 >= B.limit_ns) {
+            atomicExch(B.err, (int)LFX_TIMEOUT);
             *ok = 0;
             break;
           }
@@ -107,10 +127,10 @@ __device__ __forceinline__ bool cg_barrier(unsigned* bar, int* err, unsigned& ta
 }
 
 // the last block to leave makes the barrier ready for the next launch
-__device__ __forceinline__ void cg_leave(unsigned* bar) {
-  if (threadIdx.x == 0 && atomicAdd(bar + 1, 1u) == gridDim.x - 1) {
-    bar[0] = 0u;
-    bar[1] = 0u;
+__device__ __forceinline__ void cg_leave(const GridBar& B) {
+  if (threadIdx.x == 0 && atomicAdd(B.words + 1, 1u) == gridDim.x - 1) {
+    B.words[0] = 0u;
+    B.words[1] = 0u;
   }
 }
 
@@ -341,6 +361,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_persist(CgArgs<T> A, State* 
   __shared__ int ok;
   State c = first ? init : *S;  // every block keeps the scalars, computed alike
   if (c.done) return;
+  if (grid_failed(A.bar)) return;
   const int sub = threadIdx.x / RT, tid = threadIdx.x % RT;
   const int ch = blockIdx.x + gridDim.x * sub;  // at most one chunk a sub-group
   const bool mine = ch < A.nch;
@@ -371,7 +392,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_persist(CgArgs<T> A, State* 
   T zv[RPER];
   if (first) {
     cg_apply<T, N, EDGE>(A, A.x, cache, ncache);
-    if (!cg_barrier<CLUSTER>(A.bar, A.err, target, &ok)) return;
+    if (!cg_barrier<CLUSTER>(A.bar, target, &ok)) return;
     if (mine) {
       double a0 = 0.0, a1 = 0.0;
 #pragma unroll
@@ -393,7 +414,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_persist(CgArgs<T> A, State* 
         __stcg(part_rr + A.nch + ch, a1);
       }
     }
-    if (!cg_barrier<CLUSTER>(A.bar, A.err, target, &ok)) return;
+    if (!cg_barrier<CLUSTER>(A.bar, target, &ok)) return;
     cg_total<2>(part_rr, A.nch, sm, tot);
     c.applies = 1;
     c.r_nrm_0 = sqrt(tot[0]);
@@ -406,7 +427,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_persist(CgArgs<T> A, State* 
   }
   for (int it = 0; it < A.iters && !c.done; ++it) {
     cg_apply<T, N, EDGE>(A, A.p, cache, ncache);
-    if (!cg_barrier<CLUSTER>(A.bar, A.err, target, &ok)) return;
+    if (!cg_barrier<CLUSTER>(A.bar, target, &ok)) return;
     if (mine) {
 #pragma unroll
       for (int m = 0; m < RPER; ++m) zv[m] = m < left ? __ldcg(A.z + base + m * RT) : T(0);
@@ -417,7 +438,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_persist(CgArgs<T> A, State* 
       acc = cg_sub_sum(acc, sm);
       if (tid == 0) __stcg(part_pq + ch, acc);
     }
-    if (!cg_barrier<CLUSTER>(A.bar, A.err, target, &ok)) return;
+    if (!cg_barrier<CLUSTER>(A.bar, target, &ok)) return;
     cg_total<1>(part_pq, A.nch, sm, tot);
     c.applies += 1;
     const double alpha = c.rz / tot[0], neg_alpha = -alpha;
@@ -442,7 +463,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_persist(CgArgs<T> A, State* 
         __stcg(part_rr + A.nch + ch, a1);
       }
     }
-    if (!cg_barrier<CLUSTER>(A.bar, A.err, target, &ok)) return;
+    if (!cg_barrier<CLUSTER>(A.bar, target, &ok)) return;
     cg_total<2>(part_rr, A.nch, sm, tot);
     c.iter += 1;
     const double beta = tot[1] / c.rz;
@@ -469,7 +490,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_persist(CgArgs<T> A, State* 
     }
     if (c.iter >= c.max_iter) c.done = 1;
     if (c.done) break;
-    if (!cg_barrier<CLUSTER>(A.bar, A.err, target, &ok)) return;
+    if (!cg_barrier<CLUSTER>(A.bar, target, &ok)) return;
   }
   for (int m = 0; m < left; ++m) {
     A.x[base + m * RT] = xs[m * RT + tid];

@@ -148,7 +148,11 @@ int to_host_wait(lfx_ctx* ctx, void* host_dev, const void* dev, size_t bytes) {
                                              reinterpret_cast<int*>(ctx->h_scalars_dev + kHostErr), mark);
   ctx->launches++;
   LFX_CK(ctx, cudaGetLastError());
-  return host_wait(ctx);
+  int rc = host_wait(ctx);
+  // a bounded wait that ran out ends the solve here, not after its last iteration
+  if (!rc && *reinterpret_cast<const volatile int*>(ctx->h_scalars + kHostErr))
+    rc = lfx_ctx_check_device_error(ctx);
+  return rc;
 }
 
 void timing_end(lfx_ctx* ctx) {
@@ -276,6 +280,12 @@ int64_t lfx_ctx_launch_count(const lfx_ctx* ctx) { return ctx ? ctx->launches : 
 int lfx_ctx_set_apply_kernel(lfx_ctx* ctx, int32_t which) {
   if (!ctx || which < -1 || which > 6 || which == 2) return LFX_INVALID_ARGUMENT;
   ctx->lma_kernel = which;
+  return LFX_OK;
+}
+
+int lfx_ctx_set_wait_limit(lfx_ctx* ctx, double seconds) {
+  if (!ctx || !(seconds >= 0.0) || seconds > 60.0) return LFX_INVALID_ARGUMENT;
+  ctx->wait_ns = (unsigned long long)(seconds * 1e9);
   return LFX_OK;
 }
 

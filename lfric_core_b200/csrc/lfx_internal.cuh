@@ -52,6 +52,7 @@ struct lfx_ctx {
   double timed_ms[2] = {0.0, 0.0};
   int64_t launches = 0;  // kernels launched on this context
   int lma_kernel = -1;   // -1: per-operator choice, 0: force pipeline, 1: force gather
+  unsigned long long wait_ns = 2000000000ull;  // longest barrier wait of a persistent CG or GMRES launch
   int* d_err = nullptr;  // [0] set by a kernel whose bounded wait ran out; [2..3] grid barrier words
   // while a solver captures a CUDA graph, timed applies record into fresh
   // event pairs owned by that graph
@@ -489,7 +490,8 @@ struct HostMark {
 };
 HostMark host_next(lfx_ctx* ctx);
 int host_wait(lfx_ctx* ctx);
-// bytes to the host with the device error flag, and waits for them
+// bytes to the host with the device error flag, and waits for them; LFX_TIMEOUT
+// (and flag and barrier words ready for the next launch) when it was set
 int to_host_wait(lfx_ctx* ctx, void* host_dev, const void* dev, size_t bytes);
 void timing_begin(lfx_ctx* ctx, int32_t precision);
 void timing_end(lfx_ctx* ctx);

@@ -27,8 +27,7 @@ struct MgsArgs {
   double *inv_hn, *sig;
   int* applies;
   double* partials;  // 2 nch
-  unsigned* bar;     // {arrivals, blocks gone}, zero between launches
-  int* err;
+  GridBar bar;
   const int* skip;
 };
 
@@ -63,6 +62,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) mgs_persist(const MgsArgs<T> A)
   __shared__ double sm[kCgSubs * (RT / 32)], tot[2];
   __shared__ int ok;
   if (*((volatile const int*)A.skip)) return;
+  if (grid_failed(A.bar)) return;
   T* ws = reinterpret_cast<T*>(mgs_smem);
   const int sub = threadIdx.x / RT, tid = threadIdx.x % RT, lane = threadIdx.x & 31;
   const int warp = tid >> 5;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) mgs_persist(const MgsArgs<T> A)
       }
       if (q1 < cnt) asm volatile("bar.sync %0, %1;" ::"r"(1 + sub), "n"(RT) : "memory");
     }
-    if (!cg_barrier<false>(A.bar, A.err, target, &ok)) return;
+    if (!cg_barrier<false>(A.bar, target, &ok)) return;
     cg_total<1>(part, A.nch, sm, tot);
     const double t = tot[0];
     if (ph < A.iv) {

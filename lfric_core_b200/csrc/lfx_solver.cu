@@ -689,8 +689,7 @@ int cg_run_persist(lfx_solver* s, const CgShape& q, T* x, const T* b) {
   A.z = (T*)s->work[2];
   A.dg = (const T*)s->prec->rdiag;
   A.partials = ctx->d_partials;
-  A.bar = ctx->d_ticket + 1;
-  A.err = ctx->d_err;
+  A.bar = grid_bar(ctx);
   A.iters = kCgItersPerLaunch;
   A.maxg = L->max_groups;
   A.lw = q.lw;
@@ -698,9 +697,8 @@ int cg_run_persist(lfx_solver* s, const CgShape& q, T* x, const T* b) {
     const DevState init = *s->h_state;  // (as init_state left it, for the first launch)
     int rc = L->ndf_from == 6 ? cg_persist_form<T, 6>(ctx, A, s->d_state, init, first, q)
                               : cg_persist_form<T, 8>(ctx, A, s->d_state, init, first, q);
+    // (a barrier that ran out leaves the state as it was: read_state reports it)
     if (!rc) rc = read_state(s);
-    // a barrier that ran out leaves the state as it was
-    if (!rc && !s->h_state->done) rc = lfx_ctx_check_device_error(ctx);
     if (rc || s->h_state->done) return rc;
   }
 }
@@ -1245,8 +1243,7 @@ int gmres_run(lfx_solver* s, T* x, const T* b, bool one_cycle = false) {
         A.sig = &sig[iv];
         A.applies = &S->applies;
         A.partials = ctx->d_partials;
-        A.bar = ctx->d_ticket + 1;
-        A.err = ctx->d_err;
+        A.bar = grid_bar(ctx);
         A.skip = askip;
         if ((q = mgs_launch(ctx, A))) return q;
         continue;
@@ -1706,9 +1703,7 @@ int lfx_solver_apply(lfx_solver* s, lfx_vec* x, const lfx_vec* b, lfx_solve_info
     if (!rc) fill_info(s, info);  // (each of them ends with the state read)
   }
   if (ctx->time_applies) drain_timing(ctx);
-  // (the device error flag came with the last state or norm)
-  if (!rc && *reinterpret_cast<const volatile int*>(ctx->h_scalars + kHostErr))
-    rc = lfx_ctx_check_device_error(ctx);
+  // (a wait that ran out was reported by the look at the state or norm after it)
   if (rc) {
     info->status = rc;
     return rc;

@@ -91,6 +91,7 @@ _SIGS = [
     ("lfx_ctx_launch_count", [vp], C.c_int64),
     ("lfx_ctx_set_apply_kernel", [vp, C.c_int32], C.c_int),
     ("lfx_ctx_check_device_error", [vp], C.c_int),
+    ("lfx_ctx_set_wait_limit", [vp, C.c_double], C.c_int),
     ("lfx_vec_create", [vp, C.c_int32, i64p, C.c_int32, C.POINTER(vp)], C.c_int),
     ("lfx_vec_duplicate", [vp, C.POINTER(vp)], C.c_int),
     ("lfx_vec_destroy", [vp], C.c_int),
@@ -273,6 +274,10 @@ class Context:
 
     def check_device_error(self):
         self.check(self.L.lfx_ctx_check_device_error(self.h))
+
+    def set_wait_limit(self, seconds):
+        """Longest barrier wait of the persistent CG and GMRES launches."""
+        self.check(self.L.lfx_ctx_set_wait_limit(self.h, float(seconds)))
 
     def close(self):
         if getattr(self, "h", None):
