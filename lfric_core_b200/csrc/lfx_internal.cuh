@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "lfx.h"
+#include "lfx_kernel_attrs.h"
 
 // a start/stop event pair around one timed operator apply
 struct TimedPair {
@@ -51,6 +52,7 @@ struct lfx_ctx {
   int64_t timed_launches[2] = {0, 0};
   double timed_ms[2] = {0.0, 0.0};
   int64_t launches = 0;  // kernels launched on this context
+  lfx::KernelAttrs kernels;
   int lma_kernel = -1;   // -1: per-operator choice, 0: force pipeline, 1: force gather
   unsigned long long wait_ns = 2000000000ull;  // longest barrier wait of a persistent CG or GMRES launch
   int* d_err = nullptr;  // [0] set by a kernel whose bounded wait ran out; [2..3] grid barrier words

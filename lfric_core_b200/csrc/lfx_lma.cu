@@ -1869,12 +1869,7 @@ TmaShape pipe_default(const lfx_op* op) {
 template <class T, int N, int IPL, int NP>
 void launch_pipe_t(lfx_ctx* ctx, const lfx_op* op, const LayoutArgs& A, const TmaShape& ts,
                    const void* x, void* y, const void* b, const int* skip) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(lma_pipe<T, N, IPL, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kTmaSmemMax);
-    attr = true;
-  }
+  ctx->kernels.allow_smem((const void*)lma_pipe<T, N, IPL, NP>, kTmaSmemMax);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lma_pipe<T, N, IPL, NP>, 32 * ts.warps,
                                                 ts.smem);
@@ -1916,12 +1911,7 @@ void launch_pipe(lfx_ctx* ctx, const lfx_op* op, const LayoutArgs& A, const TmaS
 template <class T, int N>
 void launch_tma(lfx_ctx* ctx, const lfx_op* op, const LayoutArgs& A, const TmaShape& ts,
                 const void* x, void* y, const void* b, const int* skip) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(lma_tma<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kTmaSmemMax);
-    attr = true;
-  }
+  ctx->kernels.allow_smem((const void*)lma_tma<T, N>, kTmaSmemMax);
   // persistent warps: one resident wave of blocks, each warp walking its
   // entity columns with `stages` of them in flight
   int per_sm = 0;
@@ -1942,17 +1932,23 @@ bool fetch_ok(const lfx_op* op) {
          (L->ndf_from == 1 || L->ndf_from == 6 || L->ndf_from == 8);
 }
 
+// blocks of 256 threads an SM holds of a kernel without dynamic shared memory
+template <class K>
+int blocks_per_sm(lfx_ctx* ctx, K* kern) {
+  return ctx->kernels.once((const void*)kern, [=] {
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, 0);
+    return std::max(n, 1);
+  });
+}
+
 // one resident wave of blocks: each warp walks its columns with the
 // descriptors of the next kFetchDepth in flight. variant 0 caps registers for
 // 3 blocks of 256 per SM, variant 1 for 4 (FP32) / 2 (FP64).
 template <class T, int N, int MINB>
 void launch_fetch_t(lfx_ctx* ctx, const lfx_op* op, const LayoutArgs& A, const void* x, void* y,
                     const void* b, const int* skip) {
-  static int per_sm = 0;
-  if (!per_sm) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lma_fetch<T, N, MINB>, 256, 0);
-    if (per_sm < 1) per_sm = 1;
-  }
+  const int per_sm = blocks_per_sm(ctx, lma_fetch<T, N, MINB>);
   const int grid = (int)std::min<int64_t>(((int64_t)A.nent + 7) / 8, (int64_t)ctx->num_sms * per_sm);
   lma_fetch<T, N, MINB><<<grid, 256, 0, ctx->stream>>>(A, (const T*)op->mat, (const T*)x, (T*)y,
                                                         (const T*)b, skip);
@@ -1993,12 +1989,7 @@ void launch_cells_t(lfx_ctx* ctx, const lfx_op* op, const void* x, void* y, cons
   const size_t smem = (size_t)kCellWarps * S * sb;
   int per_sm = 1;
   if constexpr (S > 0) {
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(lma_cells_pipe<T, N, SYM, S, RESID, CANON>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmemMax);
-      attr = true;
-    }
+    ctx->kernels.allow_smem((const void*)lma_cells_pipe<T, N, SYM, S, RESID, CANON>, kCellSmemMax);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lma_cells_pipe<T, N, SYM, S, RESID, CANON>,
                                                   32 * kCellWarps, smem);
     if (per_sm < 1) per_sm = 1;
@@ -2137,11 +2128,7 @@ void launch_ring_t(lfx_ctx* ctx, const lfx_op* op, int stages, int warps, const 
   for (int k = 0; k <= R.ncol; ++k) R.cs[k] = L->colour_start[k];
   const size_t smem = ring_smem_bytes(op, stages, warps);
   auto kern = lma_cells_ring<T, N, SYM, D, RESID, CANON>;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRingSmemMax);
-    attr = true;
-  }
+  ctx->kernels.allow_smem((const void*)kern, kRingSmemMax);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem);
   if (per_sm < 1) per_sm = 1;
@@ -2440,11 +2427,7 @@ static int make_tdesc(lfx_ctx* ctx, const lfx_lma_layout* L, lfx_lma_layout* T) 
 template <class T, int NJ>
 static void launch_faces_t(lfx_ctx* ctx, const lfx_op* op, const lfx_lma_layout* L,
                            const lfx_lma_layout* TL, const void* x, void* y) {
-  static int per_sm = 0;
-  if (!per_sm) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lma_faces_t<T, NJ>, 256, 0);
-    if (per_sm < 1) per_sm = 1;
-  }
+  const int per_sm = blocks_per_sm(ctx, lma_faces_t<T, NJ>);
   const int grid = (int)std::max<int64_t>(
       1, std::min<int64_t>(((int64_t)TL->nent + 7) / 8, (int64_t)ctx->num_sms * per_sm));
   lma_faces_t<T, NJ><<<grid, 256, 0, ctx->stream>>>(TL->nent, L->nlayers, op->blk, TL->tdesc,

@@ -1789,22 +1789,12 @@ int gram(lfx_mrhs* m, const float* U, const float* V0, const float* V1, const fl
   lfx_ctx* ctx = m->ctx;
   const int64_t n = m->undf;
   if (m->gram_tc) {
-    static bool attr = false;
-    if (!attr) {
-      LFX_CK(ctx, cudaFuncSetAttribute(bcg_gram_tc<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)tc_gram_smem<NV>()));
-      attr = true;
-    }
+    LFX_CK(ctx, ctx->kernels.allow_smem((const void*)bcg_gram_tc<NV>, tc_gram_smem<NV>()));
     bcg_gram_tc<NV><<<m->bgrid, kTcThreads, tc_gram_smem<NV>(), ctx->stream>>>(n, U, V0, V1,
                                                                                vscale, m->bpart, st);
   } else {
     constexpr size_t smem = ChunkRing<1 + NV, 4>::BYTES;
-    static bool sattr = false;
-    if (!sattr) {
-      LFX_CK(ctx, cudaFuncSetAttribute(bcg_gram_s<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
-      sattr = true;
-    }
+    LFX_CK(ctx, ctx->kernels.allow_smem((const void*)bcg_gram_s<NV>, smem));
     bcg_gram_s<NV><<<m->bgrid, 256, smem, ctx->stream>>>(n, U, V0, V1, vscale, m->bpart, st);
   }
   const int ne = NV * kBS * kBS;
@@ -1817,8 +1807,7 @@ int gram(lfx_mrhs* m, const float* U, const float* V0, const float* V1, const fl
 int ensure_bcg(lfx_mrhs* m) {
   if (m->bcg) return LFX_OK;
   lfx_ctx* ctx = m->ctx;
-  LFX_CK(ctx, cudaFuncSetAttribute(bcg_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)kBcgSmallSmem));
+  LFX_CK(ctx, ctx->kernels.allow_smem((const void*)bcg_small, kBcgSmallSmem));
   m->bgrid = ctx->num_sms * 2;
   int rc = dmalloc(ctx, (void**)&m->w32, (size_t)m->undf * m->nrhs * 4);
   if (!rc) rc = dmalloc(ctx, (void**)&m->bcg, sizeof(BcgSmall));
@@ -1833,12 +1822,7 @@ int ensure_bcg(lfx_mrhs* m) {
 template <int MODE>
 auto upd_launch(lfx_ctx* ctx, int G) {
   using RG = ChunkRing<UpdOps<MODE>::NA, UpdOps<MODE>::S>;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(bcg_update_s<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)RG::BYTES);
-    attr = true;
-  }
+  ctx->kernels.allow_smem((const void*)bcg_update_s<MODE>, RG::BYTES);
   return [ctx, G](int64_t n, const float* A0, const float* A1, float* Y0, float* Y1,
                   const float* dinv, const BcgSmall* st, int skip_p, double* partials) {
     bcg_update_s<MODE><<<G, 256, RG::BYTES, ctx->stream>>>(n, A0, A1, Y0, Y1, dinv, st, skip_p,

@@ -450,12 +450,7 @@ constexpr int kJacobiBlocksPerSm = 4;
 template <class T, bool SF>
 void launch_staged(lfx_ctx* ctx, const lfx_prec* p, const T* x, T* y, size_t smem,
                    const int* skip) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(cma_prec_staged<T, SF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kStageSmemMax);
-    attr = true;
-  }
+  ctx->kernels.allow_smem((const void*)cma_prec_staged<T, SF>, kStageSmemMax);
   const int tb = (p->ncell_2d + kStageCols - 1) / kStageCols;
   if (p->rdiag && p->zero_sentinel) {
     // the column sweeps, then the Jacobi rows as a programmatic dependent

@@ -468,10 +468,12 @@ __global__ void __launch_bounds__(kCgsThreads) cgs_update_f4(int64_t n, VecPtrs 
 
 // blocks of a float4 Gram-Schmidt kernel resident on the GPU at once
 template <class K>
-int resident_blocks(const lfx_ctx* ctx, K kernel) {
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kCgsThreads, 0);
-  return ctx->num_sms * std::max(per_sm, 1);
+int resident_blocks(lfx_ctx* ctx, K* kernel) {
+  return ctx->kernels.once((const void*)kernel, [=] {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kCgsThreads, 0);
+    return ctx->num_sms * std::max(per_sm, 1);
+  });
 }
 
 bool quad_aligned(const VecPtrs& vp, int nr, const void* w) {
@@ -486,9 +488,7 @@ int cgs_step_f4(lfx_ctx* ctx, int64_t n, const VecPtrs& vp, float* w, float* out
                 double* nhcol, const double* sig, int prev, Fin fin, const int* skip) {
   // one resident wave, and at most one block per 2048 values (the partials
   // scratch holds nchunks(n) values per sum)
-  static int gd = 0, gu = 0;
-  if (!gd) gd = resident_blocks(ctx, cgs_dots_f4<NR>);
-  if (!gu) gu = resident_blocks(ctx, cgs_update_f4<NR, Fin>);
+  const int gd = resident_blocks(ctx, cgs_dots_f4<NR>), gu = resident_blocks(ctx, cgs_update_f4<NR, Fin>);
   const int64_t cap = std::max<int64_t>(1, nchunks(n));
   cgs_dots_f4<NR><<<(int)std::min<int64_t>(gd, cap), kCgsThreads, 0, ctx->stream>>>(
       n, vp, w, hcol, nhcol, sig, prev, ctx->d_partials, ctx->d_ticket, skip);
@@ -599,14 +599,7 @@ int cg_persist_launch(lfx_ctx* ctx, CgArgs<T> A, DevState* S, const DevState& in
   const size_t vec = (size_t)((A.nch + grid - 1) / grid) * cg_chunk_bytes<T>();
   const size_t per = 32 >> A.lw, cols = ((size_t)(A.nent + grid - 1) / grid + per - 1) / per * per;
   A.smem = (int)std::min(kCgSmemMax, vec + cols * A.maxg * cg_group_bytes<T, N>(A.nl));
-  static bool attr = false;
-  if (!attr) {
-    LFX_CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kCgSmemMax));
-    if (CLUSTER)
-      LFX_CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    attr = true;
-  }
+  LFX_CK(ctx, ctx->kernels.allow_smem((const void*)kern, kCgSmemMax));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kCgThreads);
@@ -628,13 +621,12 @@ int cg_persist_launch(lfx_ctx* ctx, CgArgs<T> A, DevState* S, const DevState& in
   return LFX_OK;
 }
 
-// whether the device holds a cluster of kCgCluster such blocks
+// whether the device holds a cluster of kCgCluster such blocks (and allows it)
 template <class T, int N, bool EDGE>
-bool cg_cluster_fits(const lfx_ctx* ctx) {
-  static int fits = -1;
-  if (fits < 0) {
-    auto kern = cg_persist<T, N, true, EDGE, DevState>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgSmemMax);
+bool cg_cluster_fits(lfx_ctx* ctx) {
+  auto kern = cg_persist<T, N, true, EDGE, DevState>;
+  return ctx->kernels.once((const void*)kern, [=] {
+    ctx->kernels.allow_smem((const void*)kern, kCgSmemMax);
     cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kCgCluster);
@@ -648,10 +640,10 @@ bool cg_cluster_fits(const lfx_ctx* ctx) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int n = 0;
-    fits = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
+    const bool fits = cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
     cudaGetLastError();
-  }
-  return fits == 1;
+    return fits ? 1 : 0;
+  }) == 1;
 }
 
 template <class T, int N>
@@ -1011,12 +1003,7 @@ __global__ void __launch_bounds__(256) gmres_xupdate(int64_t n, VecPtrs vp, cons
 
 template <class T>
 int mgs_launch(lfx_ctx* ctx, const MgsArgs<T>& A) {
-  static bool attr = false;
-  if (!attr) {
-    LFX_CK(ctx, cudaFuncSetAttribute(mgs_persist<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kMgsSmemMax));
-    attr = true;
-  }
+  LFX_CK(ctx, ctx->kernels.allow_smem((const void*)mgs_persist<T>, kMgsSmemMax));
   // a chunk a sub-group while there are blocks for it
   const int grid = std::max(1, std::min((A.nch + kCgSubs - 1) / kCgSubs, ctx->num_sms));
   cudaLaunchConfig_t cfg = {};
