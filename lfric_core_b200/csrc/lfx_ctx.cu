@@ -3,6 +3,7 @@
 #include <cstdio>
 #include <cstring>
 
+#include "lfx_host_number.h"
 #include "lfx_internal.cuh"
 
 namespace lfx {
@@ -129,14 +130,14 @@ HostMark host_next(lfx_ctx* ctx) {
 // The number arrives when every operation queued before its kernel is done. A
 // stream that ends without it (a failed launch) is reported.
 int host_wait(lfx_ctx* ctx) {
-  const volatile unsigned* p = reinterpret_cast<const volatile unsigned*>(ctx->h_scalars + kHostSeq);
+  const unsigned* p = reinterpret_cast<const unsigned*>(ctx->h_scalars + kHostSeq);
   for (unsigned spin = 1;; ++spin) {
-    if (*p == ctx->host_seq) return LFX_OK;
+    if (host_number(p) == ctx->host_seq) return LFX_OK;
     if (spin % 4096) continue;
     const cudaError_t e = cudaStreamQuery(ctx->stream);
     if (e == cudaErrorNotReady) continue;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamQuery");
-    if (*p == ctx->host_seq) return LFX_OK;
+    if (host_number(p) == ctx->host_seq) return LFX_OK;
     return fail(ctx, LFX_CUDA_ERROR, "a result never reached the host");
   }
 }
@@ -241,9 +242,10 @@ int lfx_ctx_enable_apply_timing(lfx_ctx* ctx, int32_t enable) {
   return LFX_OK;
 }
 
-// Folds the recorded event pairs into the running totals (the stream must be
-// idle, which lfx_solver_apply guarantees on return).
+// Folds the recorded event pairs into the running totals. The stream is made idle
+// first: a solve returns when its last number is there, which is a little earlier.
 static int collect_timing(lfx_ctx* ctx) {
+  LFX_CK(ctx, cudaStreamSynchronize(ctx->stream));
   for (int i = 0; i + 1 < ctx->ev_used; i += 2) {
     float ms = 0.f;
     cudaError_t e = cudaEventElapsedTime(&ms, ctx->ev_pool[i], ctx->ev_pool[i + 1]);
@@ -259,7 +261,6 @@ static int collect_timing(lfx_ctx* ctx) {
 int lfx_ctx_apply_timing(lfx_ctx* ctx, int32_t precision, int64_t* launches, double* total_ms,
                          int32_t reset) {
   if (!ctx) return LFX_INVALID_ARGUMENT;
-  LFX_CK(ctx, cudaStreamSynchronize(ctx->stream));
   int rc = collect_timing(ctx);
   if (rc) return rc;
   const bool all = precision == 0;

@@ -163,6 +163,7 @@ void collect_timing(lfx_solver* s) {
   const int pi = s->pending;
   s->pending = -1;
   if (pi < 0 || pi >= (int)s->graphs.size() || !ctx->time_applies) return;
+  cudaStreamSynchronize(ctx->stream);
   GraphEntry* ge = &s->graphs[pi];
   for (auto& p : ge->ev) {
     float ms = 0.f;
