@@ -719,8 +719,15 @@ __device__ __noinline__ void alpha_phase(const BParams& P, BShared& sh) {
 // Where that gives every block of the largest grid 4 kChGroup chunks or more, an item
 // takes kChGroup of them (each with its own partial, so the bits stay), with one
 // block sum and one ticket an item: 256 uneven W0 slots (63 M rows, 15 424 chunks)
-// took 3388 us an iteration with a chunk an item, 3291 so (3240-3270 with chunks of
-// 16384 values, which cost the few slots above).
+// took 3388 us an iteration with a chunk an item, 3291 so.
+// Indices are 32 bits wide (a field has less than 2^31 values) and a phase without
+// sums takes a group's chunks as one run: with 64-bit indices the group's counters
+// spilled in the first phase (52 bytes; 4 now). 64 W2 slots (275 M rows) to 1e-10:
+// 238.4 -> 235.3 ms, 16 (69 M) 67.0 -> 66.1, 6 (38 M) 42.6 -> 42.1; 256 W0 slots
+// (59 M) 664 -> 663, 12 (2.5 M) 62.0 -> 61.3. With chunks of 16384 values and no
+// groups those took 232.6, 66.0, 42.3, 658 and 69.5: the largest batches pay 1 % for
+// what the few slots gain. (Sums of a group's chunks kept in shared memory and
+// added up side by side: 241.5 ms for the 64.)
 constexpr int kVStep = kBT * 4;                   // values per block step
 constexpr int kVSteps = kBSub * RCHUNK / kVStep;  // steps per chunk (4)
 static_assert(kVSteps % 2 == 0, "two steps per pass");
@@ -733,7 +740,7 @@ struct VState {
 // four consecutive values from i (zeros past n); RO: read-only during the
 // launch (non-coherent cache), else read through L2
 template <bool RO>
-__device__ __forceinline__ float4 vld(const float* a, int64_t i, int64_t n) {
+__device__ __forceinline__ float4 vld(const float* a, unsigned i, unsigned n) {
   if (i + 3 < n)
     return RO ? __ldg(reinterpret_cast<const float4*>(a + i))
               : __ldcg(reinterpret_cast<const float4*>(a + i));
@@ -743,7 +750,7 @@ __device__ __forceinline__ float4 vld(const float* a, int64_t i, int64_t n) {
   if (i + 2 < n) v.z = RO ? __ldg(a + i + 2) : __ldcg(a + i + 2);
   return v;
 }
-__device__ __forceinline__ void vst(float* a, int64_t i, int64_t n, float4 v) {
+__device__ __forceinline__ void vst(float* a, unsigned i, unsigned n, float4 v) {
   if (i + 3 < n) {
     __stcg(reinterpret_cast<float4*>(a + i), v);
     return;
@@ -760,7 +767,7 @@ struct DF4 {
   float4 f;
 };
 template <bool RO>
-__device__ __forceinline__ D4 vldd(const double* a, int64_t i, int64_t n) {
+__device__ __forceinline__ D4 vldd(const double* a, unsigned i, unsigned n) {
   D4 r;
   if (i + 3 < n) {
     const double2 lo = RO ? __ldg(reinterpret_cast<const double2*>(a + i))
@@ -774,7 +781,7 @@ __device__ __forceinline__ D4 vldd(const double* a, int64_t i, int64_t n) {
   for (int c = 0; c < 4; ++c) r.v[c] = i + c < n ? (RO ? __ldg(a + i + c) : __ldcg(a + i + c)) : 0.0;
   return r;
 }
-__device__ __forceinline__ void vstd(double* a, int64_t i, int64_t n, const D4& r) {
+__device__ __forceinline__ void vstd(double* a, unsigned i, unsigned n, const D4& r) {
   if (i + 3 < n) {
     __stcg(reinterpret_cast<double2*>(a + i), make_double2(r.v[0], r.v[1]));
     __stcg(reinterpret_cast<double2*>(a + i + 2), make_double2(r.v[2], r.v[3]));
@@ -805,16 +812,17 @@ __device__ __noinline__ void vec_phase(const BParams& P, BShared& sh, Pred pred,
     V.fresh = __ldcg(&Sg->fresh);
     V.alpha = (float)__ldcg(&Sg->alpha);
     V.beta = (float)__ldcg(&Sg->beta);
-    const int64_t n = D.n;
+    const unsigned n = (unsigned)D.n;  // (below 2^31: 64-bit indices spill in the first phase)
     const int ch0 = item.y * P.chgrp, nk = min(P.chgrp, D.nch - ch0);
-    for (int k = 0; k < nk; ++k) {
+    const int reps = NR > 0 ? nk : 1, steps = NR > 0 ? kVSteps : nk * kVSteps;
+    for (int k = 0; k < reps; ++k) {
       double acc[NR > 0 ? NR : 1];
 #pragma unroll
       for (int r = 0; r < (NR > 0 ? NR : 1); ++r) acc[r] = 0.0;
-      const int64_t c0 = (int64_t)(ch0 + k) * (kBSub * RCHUNK);
-      for (int stp = 0; stp < kVSteps; stp += 2) {
-        if (c0 + (int64_t)stp * kVStep >= n) break;  // block-uniform
-        const int64_t i0 = c0 + (int64_t)stp * kVStep + 4 * threadIdx.x, i1 = i0 + kVStep;
+      const unsigned c0 = (unsigned)(ch0 + k) * (kBSub * RCHUNK);
+      for (int stp = 0; stp < steps; stp += 2) {
+        if (c0 + stp * kVStep >= n) break;  // block-uniform
+        const unsigned i0 = c0 + stp * kVStep + 4 * threadIdx.x, i1 = i0 + kVStep;
         const auto a = ld(D, i0, n);
         const auto b = ld(D, i1, n);
         if (i0 < n) op(D, V, i0, n, a, acc);
@@ -1101,12 +1109,12 @@ __global__ void __launch_bounds__(kBT, kMaxBps) batch_kernel(const BParams* __re
     int* need = P.need + it;
     vec_phase<2>(
         P, sh, [](int ph, int) { return ph_run(ph); },
-        [](const BSlot& D, int64_t i, int64_t n) {
+        [](const BSlot& D, unsigned i, unsigned n) {
           return W5<float4>{vld<false>(D.xc, i, n), vld<false>(D.p, i, n), vld<false>(D.r, i, n),
                             vld<false>(D.z, i, n),
                             D.cma ? make_float4(1.f, 1.f, 1.f, 1.f) : vld<true>(D.diag, i, n)};
         },
-        [](const BSlot& D, const VState& S, int64_t i, int64_t n, const W5<float4>& v, double* a) {
+        [](const BSlot& D, const VState& S, unsigned i, unsigned n, const W5<float4>& v, double* a) {
           float xc[4], p[4], r[4], z[4], d[4];
           f4a(v.a, xc); f4a(v.b, p); f4a(v.c, r); f4a(v.d, z); f4a(v.e, d);
 #pragma unroll
@@ -1139,10 +1147,10 @@ __global__ void __launch_bounds__(kBT, kMaxBps) batch_kernel(const BParams* __re
       auto resid = [](int ph, int fl) { return ph == PH_INIT || (ph == PH_RUN && fl); };
       vec_phase<0>(
           P, sh, resid,
-          [](const BSlot& D, int64_t i, int64_t n) {
+          [](const BSlot& D, unsigned i, unsigned n) {
             return DF4{vldd<false>(D.x, i, n), vld<false>(D.xc, i, n)};
           },
-          [](const BSlot& D, const VState& S, int64_t i, int64_t n, const DF4& v, double*) {
+          [](const BSlot& D, const VState& S, unsigned i, unsigned n, const DF4& v, double*) {
             if (S.phase != PH_INIT) {
               float xc[4];
               f4a(v.f, xc);
@@ -1163,10 +1171,10 @@ __global__ void __launch_bounds__(kBT, kMaxBps) batch_kernel(const BParams* __re
         }
       vec_phase<2>(
           P, sh, resid,
-          [](const BSlot& D, int64_t i, int64_t n) {
+          [](const BSlot& D, unsigned i, unsigned n) {
             return DF4{vldd<false>(D.r64, i, n), vld<true>(D.diag, i, n)};
           },
-          [](const BSlot& D, const VState&, int64_t i, int64_t n, const DF4& v, double* a) {
+          [](const BSlot& D, const VState&, unsigned i, unsigned n, const DF4& v, double* a) {
             float d[4], r[4];
             f4a(v.f, d);
 #pragma unroll
@@ -1220,11 +1228,11 @@ __global__ void __launch_bounds__(kBT, kMaxBps) batch_kernel(const BParams* __re
       if (!grid_sync(P, sh)) return;
       vec_phase<1>(
           P, sh, [](int ph, int) { return ph_run(ph); },
-          [](const BSlot& D, int64_t i, int64_t n) {
+          [](const BSlot& D, unsigned i, unsigned n) {
             if (!D.cma) return V3<float4>{};
             return V3<float4>{vld<false>(D.r, i, n), vld<true>(D.diag, i, n), vld<false>(D.z, i, n)};
           },
-          [](const BSlot& D, const VState&, int64_t i, int64_t n, const V3<float4>& v, double* a) {
+          [](const BSlot& D, const VState&, unsigned i, unsigned n, const V3<float4>& v, double* a) {
             if (!D.cma) return;
             // rows with a non-zero diagonal are Jacobi rows; the column rows
             // (written by the sweeps) carry a zero in the Jacobi diagonal
@@ -1251,11 +1259,11 @@ __global__ void __launch_bounds__(kBT, kMaxBps) batch_kernel(const BParams* __re
     // ---- P: p = z + beta p (p = z for a slot that just started)
     vec_phase<0>(
         P, sh, [](int ph, int) { return ph_run(ph); },
-        [](const BSlot& D, int64_t i, int64_t n) {
+        [](const BSlot& D, unsigned i, unsigned n) {
           return V3<float4>{vld<false>(D.p, i, n), D.cma ? vld<false>(D.z, i, n) : vld<false>(D.r, i, n),
                             D.cma ? make_float4(1.f, 1.f, 1.f, 1.f) : vld<true>(D.diag, i, n)};
         },
-        [](const BSlot& D, const VState& S, int64_t i, int64_t n, const V3<float4>& v, double*) {
+        [](const BSlot& D, const VState& S, unsigned i, unsigned n, const V3<float4>& v, double*) {
           float p[4], zr[4], d[4];
           f4a(v.a, p); f4a(v.b, zr); f4a(v.c, d);
 #pragma unroll
