@@ -585,10 +585,21 @@ CgShape cg_shape(const lfx_solver* s) {
   const int64_t warps = (L->nent + cols - 1) / cols, all = kCgThreads / 32;
   q.cluster = warps <= kCgCluster * all && nch <= (int64_t)kCgSubs * kCgCluster;
   // half-full blocks before a second column a warp
-  q.grid = q.cluster ? kCgCluster
-                     : (int)std::min<int64_t>(std::max((nch + kCgSubs - 1) / kCgSubs,
-                                                       (warps + all / 2 - 1) / (all / 2)),
-                                              ctx->num_sms);
+  const int64_t least = (nch + kCgSubs - 1) / kCgSubs, want = (warps + all / 2 - 1) / (all / 2);
+  q.grid = q.cluster ? kCgCluster : (int)std::min<int64_t>(std::max(least, want), ctx->num_sms);
+  // A block takes a whole SM, so solves of several contexts run side by side only
+  // where their grids fit together. Columns of more than 32 rows gain least from
+  // this form, and two such solves lost by queueing: where half the device has
+  // warps enough for every column it is all they take. A solve by one, two and four
+  // contexts at once, in us (launch per phase; whole device; half): C10 x 40 3357,
+  // 1824, 991; 2481, 2499, 2461; 2539, 1326, 1297. C12 x 70 5845, 3303, 1944; 4804,
+  // 4782, 4785; 4990, 2505, 2508. Not taken for lower columns, where two solves in a
+  // queue are no slower than before and half a device costs one of them more: C16 x
+  // 12 3399, 1819, 1013; 1443, 1417, 1412; 1528, 780, 762; C24 x 20 6139, 3790, 2554;
+  // 3114, 3093, 3152; 4121, 2078, 2089. (The cluster's solves run side by side: C8 x 6
+  // 1682, 867, 452; 605, 321, 159.)
+  if (!q.cluster && L->max_h > 32 && want < ctx->num_sms)
+    q.grid = (int)std::max<int64_t>(least, std::min<int64_t>(want, ctx->num_sms / 2));
   return q;
 }
 
