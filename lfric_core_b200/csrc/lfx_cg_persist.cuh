@@ -3,13 +3,13 @@
 // the launch per phase, so the same bits.
 //
 // A small solve is all latency: an iteration of five launches inside a CUDA
-// graph takes 24.2 us at C8 x 6 (2 702 dofs) and 29.3 us at C24 x 20 (72 618
+// graph takes 23.7 us at C8 x 6 (2 702 dofs) and 31.8 us at C24 x 20 (72 618
 // dofs, the matrix in L2), of which the bytes would take under 1 and 6 us.
 // Here the blocks stay resident, keep p, r, x and the diagonal of their chunks
 // in shared memory, and the records and matrix rows of as many of their dof
 // columns as fit beside them; they meet at a barrier where a launch ended
-// (four an iteration). Whole solves, FP64, B200: C8 x 6 (67 iterations) 1620 ->
-// 609 us, C24 x 20 (192) 5630 -> 3127 us, C37 x 23 (263) 12.4 -> 7.5 ms. What is
+// (four an iteration). Whole solves, FP64, B200: C8 x 6 (67 iterations) 1390-1590 ->
+// 598 us, C24 x 20 (192) 6100 -> 3141 us, C37 x 23 (263) 12.4 -> 6.9 ms. What is
 // left is latency: 15 k cycles of 31 k at C24 x 20 are the gather (two passes of
 // columns a warp, the second's matrix from L2), a grid barrier takes 2 to 3 k
 // (0.6 to 1 k the cluster's), the two reductions with their division and root

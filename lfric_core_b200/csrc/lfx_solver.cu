@@ -573,10 +573,15 @@ CgShape cg_shape(const lfx_solver* s) {
   if (s->prec->kind != PREC_DIAG || ctx->time_applies || ctx->lma_kernel >= 0) return q;
   if (!L->full_cover || !L->ent_pack || L->max_nrec > 2 || (L->ndf_from != 6 && L->ndf_from != 8))
     return q;
-  // Up to a matrix the size of L2, which the gather rereads: C48 x 30 FP32 (106
-  // MB) 46.7 us an iteration by launches, 35.7 here; FP64 (212 MB) 67.5 and 66.8,
-  // and 54 by launches of the cell scatter.
-  if (s->op->mat_bytes > (size_t)ctx->l2_bytes) return q;
+  // Up to a matrix that L2 keeps from one gather to the next. Whole solves in ms, by
+  // launches (of the cell scatter) and here, W0 FP64 unless said, L2 132 MB: columns
+  // of up to 32 rows, matrix of 74 MB (FP32) 7.2, 5.3; 97 MB 10.0, 7.3; 100 MB 10.2,
+  // 6.5; 113 MB 13.5, 13.0; 119 MB 13.7, 11.8; 123 MB 10.8, 11.2. Higher columns take
+  // a cell at a time here: 28 MB (FP32) 3.1, 2.2; 61 MB 7.2, 6.3; 86 MB 8.9, 8.9; 94
+  // MB (FP32) 7.9, 6.8; 97 MB (FP32) 7.9, 8.2; 106 MB 9.1, 10.7; 124 MB (C24 x 70)
+  // 11.9, 19.1.
+  const size_t l2 = (size_t)ctx->l2_bytes;
+  if (s->op->mat_bytes > (L->max_h > 32 ? l2 / 4 * 3 : l2 / 10 * 9)) return q;
   const int64_t nch = nchunks(s->n);
   if (nch < 1 || nch > (int64_t)kCgSubs * ctx->num_sms) return q;
   while (q.lw > 3 && L->max_h <= 1 << (q.lw - 1)) --q.lw;
