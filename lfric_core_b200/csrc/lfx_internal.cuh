@@ -315,9 +315,10 @@ struct lfx_lma_layout {
   int refcount = 1;
   std::vector<int32_t> rank;         // colour-loop position of every cell
   lfx_lma_layout* tlay = nullptr;    // from-space layout for the transpose apply
-  // a from-space layout whose columns have at most two records: three int4 a
-  // column, {base, height, records, 0} and per record, in the order of the
-  // transpose apply, {cell, df * nlayers, offset, first to-space dof of the cell}
+  // a from-space layout whose columns have at most two records, of operators with
+  // one to-space dof a cell: three int4 a column, {base, height, records, 0} and per
+  // record, in the order of the transpose apply, {cell, df * nlayers, offset, first
+  // to-space dof of the cell}
   int4* tdesc = nullptr;
   // cell-scatter plan (square operators on one dofmap whose dof columns each
   // get the same records from every cell that touches them, at most two per

@@ -761,19 +761,19 @@ __global__ void lma_gather_t(LayoutArgs A, int max_off, int blk, const T* __rest
   }
 }
 
-// The same for from-space columns of at most two records (faces): every operand's
-// address comes from one 48-byte descriptor, the next column's is loaded while a
-// column is worked on, and 64 levels' loads go out before the first sum. NJ: the
-// to-space ndf. D^T of the W2 divergence at C48 x 70 FP64 (78 MB, 12 us at 6.5
-// TB/s): 46 us by the general form (five dependent loads a row), 23 us here in one
-// resident wave (29 with eight blocks an SM, of which five fit).
-template <class T, int NJ>
+// The same for from-space columns of at most two records (faces) and one to-space
+// dof a cell: every operand's address comes from one 48-byte descriptor, the next
+// column's is loaded while a column is worked on, and 64 levels' loads go out before
+// the first sum. D^T of the W2 divergence, alone, general form and this one: C24 x 20
+// FP64 7.1 -> 6.2 us, C48 x 30 16.6 -> 10.5, C48 x 70 (78 MB, 12 us at 6.5 TB/s) 40.3
+// -> 19.1, C96 x 70 FP32 139.8 -> 43.3, in one resident wave. Not for six to-space
+// dofs, whose twelve rows a column overrun the registers: the square W2 operator at
+// C96 x 70 FP32 took 735 us so, 275 by the general form.
+template <class T>
 __global__ void __launch_bounds__(256) lma_faces_t(int nent, int nl, int blk,
                                                    const int4* __restrict__ td,
                                                    const T* __restrict__ M,
-                                                   const T* __restrict__ x,
-                                                   const int32_t* __restrict__ map_to,
-                                                   T* __restrict__ y) {
+                                                   const T* __restrict__ x, T* __restrict__ y) {
   const int lane = threadIdx.x & 31;
   const int nw = (int)((gridDim.x * blockDim.x) >> 5);
   int e = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -788,43 +788,32 @@ __global__ void __launch_bounds__(256) lma_faces_t(int nent, int nl, int blk,
       r0 = __ldg(t + 1);
       r1 = __ldg(t + 2);
     }
-    const T* Mq[2];
-    int xb[2][NJ];
+    const T *Mq[2], *xq[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      Mq[r] = M + (size_t)q[r].x * NJ * blk + q[r].y - q[r].z;
-#pragma unroll
-      for (int j = 0; j < NJ; ++j)
-        xb[r][j] = (NJ == 1 ? q[r].w : __ldg(map_to + (size_t)q[r].x * NJ + j)) - q[r].z;
+      Mq[r] = M + (size_t)q[r].x * blk + q[r].y - q[r].z;
+      xq[r] = x + q[r].w - q[r].z;
     }
-    constexpr int U = NJ == 1 ? 2 : 1;
+    constexpr int U = 2;
     for (int l0 = 0; l0 < h.y; l0 += 32 * U) {
-      T a[U][2][NJ], b[U][2][NJ];
+      T a[U][2], b[U][2];
 #pragma unroll
       for (int u = 0; u < U; ++u)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
           const int l = l0 + 32 * u + lane;
           const bool v = r < h.z && (unsigned)(l - q[r].z) < (unsigned)nl;
-#pragma unroll
-          for (int j = 0; j < NJ; ++j) {
-            a[u][r][j] = v ? __ldcs(Mq[r] + (size_t)j * blk + l) : T(0);
-            b[u][r][j] = v ? __ldg(x + xb[r][j] + l) : T(0);
-          }
+          a[u][r] = v ? __ldcs(Mq[r] + l) : T(0);
+          b[u][r] = v ? __ldg(xq[r] + l) : T(0);
         }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int l = l0 + 32 * u + lane;
         T acc = T(0);
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          if (r < h.z && (unsigned)(l - q[r].z) < (unsigned)nl) {
-            T s = T(0);
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) s = fmaT(a[u][r][j], b[u][r][j], s);
-            acc = acc + s;
-          }
-        }
+        for (int r = 0; r < 2; ++r)
+          if (r < h.z && (unsigned)(l - q[r].z) < (unsigned)nl)
+            acc = acc + fmaT(a[u][r], b[u][r], T(0));
         if (l < h.y) y[h.x + l] = acc;
       }
     }
@@ -2400,8 +2389,8 @@ int x_plus_ay_copy(lfx_ctx* ctx, int32_t precision, const void* x, double a, con
 // building them takes 0.4 ms of the first transposed apply (C48 x 70 W2: 2 MB),
 // ordering the columns' records without scratch allocations gives 0.9 back: 3.73 ms
 // without descriptors, 4.0 with them before that, 3.23 now.
-static __global__ void tdesc_build(LayoutArgs A, int max_off, int ndf_to,
-                                   const int32_t* __restrict__ map_to, int4* td) {
+static __global__ void tdesc_build(LayoutArgs A, int max_off, const int32_t* __restrict__ map_to,
+                                   int4* td) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= A.nent) return;
   int n = 0;
@@ -2411,8 +2400,7 @@ static __global__ void tdesc_build(LayoutArgs A, int max_off, int ndf_to,
     for (int o = max_off; o >= 0; --o)
       for (int r = 0; r < rec_n(pk); ++r) {
         if (rec_off(pk, r) != o || n == 2) continue;
-        td[3 * (size_t)e + 1 + n++] =
-            make_int4(c, rec_df(pk, r) * A.nlayers, o, map_to[(size_t)c * ndf_to]);
+        td[3 * (size_t)e + 1 + n++] = make_int4(c, rec_df(pk, r) * A.nlayers, o, map_to[c]);
       }
   }
   for (int q = n; q < 2; ++q) td[3 * (size_t)e + 1 + q] = make_int4(0, 0, 0, 0);
@@ -2422,33 +2410,26 @@ static __global__ void tdesc_build(LayoutArgs A, int max_off, int ndf_to,
 static int make_tdesc(lfx_ctx* ctx, const lfx_lma_layout* L, lfx_lma_layout* T) {
   const int rc = dmalloc(ctx, (void**)&T->tdesc, (size_t)T->nent * 48);
   if (rc) return rc;
-  tdesc_build<<<(T->nent + 255) / 256, 256, 0, ctx->stream>>>(args_of(T, 0), T->max_off, L->ndf_to,
-                                                              L->map_to, T->tdesc);
+  tdesc_build<<<(T->nent + 255) / 256, 256, 0, ctx->stream>>>(args_of(T, 0), T->max_off, L->map_to,
+                                                              T->tdesc);
   LFX_CK(ctx, cudaGetLastError());
   return LFX_OK;
-}
-
-// one resident wave of blocks
-template <class T, int NJ>
-static void launch_faces_t(lfx_ctx* ctx, const lfx_op* op, const lfx_lma_layout* L,
-                           const lfx_lma_layout* TL, const void* x, void* y) {
-  const int per_sm = blocks_per_sm(ctx, lma_faces_t<T, NJ>);
-  const int grid = (int)std::max<int64_t>(
-      1, std::min<int64_t>(((int64_t)TL->nent + 7) / 8, (int64_t)ctx->num_sms * per_sm));
-  lma_faces_t<T, NJ><<<grid, 256, 0, ctx->stream>>>(TL->nent, L->nlayers, op->blk, TL->tdesc,
-                                                    (const T*)op->mat, (const T*)x, L->map_to, (T*)y);
 }
 
 template <class T>
 static void launch_transpose(lfx_ctx* ctx, const lfx_op* op, const lfx_lma_layout* L,
                              const lfx_lma_layout* TL, const void* x, void* y) {
-  if (TL->tdesc && L->ndf_to == 1)
-    launch_faces_t<T, 1>(ctx, op, L, TL, x, y);
-  else if (TL->tdesc && L->ndf_to == 6)
-    launch_faces_t<T, 6>(ctx, op, L, TL, x, y);
-  else
+  if (!TL->tdesc) {
     lma_gather_t<T><<<gather_grid(ctx, TL->nent), 256, 0, ctx->stream>>>(
         args_of(TL, op->blk), TL->max_off, op->blk, (const T*)op->mat, (const T*)x, L->map_to, (T*)y);
+    return;
+  }
+  // one resident wave of blocks
+  const int grid = (int)std::max<int64_t>(
+      1, std::min<int64_t>(((int64_t)TL->nent + 7) / 8,
+                           (int64_t)ctx->num_sms * blocks_per_sm(ctx, lma_faces_t<T>)));
+  lma_faces_t<T><<<grid, 256, 0, ctx->stream>>>(TL->nent, L->nlayers, op->blk, TL->tdesc,
+                                                (const T*)op->mat, (const T*)x, (T*)y);
 }
 
 extern "C" {
@@ -2812,8 +2793,8 @@ int lfx_op_apply_transpose(lfx_op* op, const lfx_vec* x, lfx_vec* y) {
     }
     L->tlay = T;
     // (without memory for the descriptors the general form does the work)
-    if (T->nent && T->max_blocks <= 2 && (L->ndf_to == 1 || L->ndf_to == 6) &&
-        (rc = make_tdesc(ctx, L, T)) && rc != LFX_OUT_OF_MEMORY)
+    if (T->nent && T->max_blocks <= 2 && L->ndf_to == 1 && (rc = make_tdesc(ctx, L, T)) &&
+        rc != LFX_OUT_OF_MEMORY)
       return rc;
   }
   lfx_lma_layout* T = L->tlay;
