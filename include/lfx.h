@@ -368,7 +368,8 @@ int lfx_refined_solver_create(lfx_ctx* ctx, lfx_op* op64, lfx_solver* inner,
                               lfx_solver** out);
 
 /* Per-kernel device timing of the operator apply: when enabled, CUDA events
- * bracket every LMA apply launched on this context; lfx_ctx_apply_timing
+ * bracket every LMA apply launched on this context (a small CG solve, otherwise one
+ * launch, then runs a launch per phase: its applies are those of that form); lfx_ctx_apply_timing
  * returns the count and total milliseconds of the applies of the given
  * storage precision (0 = all) accumulated since the last reset. */
 int lfx_ctx_enable_apply_timing(lfx_ctx* ctx, int32_t enable);
@@ -492,7 +493,10 @@ int lfx_mrhs_autotune(lfx_mrhs* m, int32_t reps, int32_t* levels_per_block, floa
 enum { LFX_MRHS_PER_RHS_CG = 0, LFX_MRHS_BLOCK_CG = 1 };
 typedef struct {
   double r_tol;      /* per right-hand side: ||b - A x|| <= r_tol ||b - A x0|| */
-  double inner_tol;  /* each inner FP32 solve reduces its residual by this */
+  /* each inner FP32 solve reduces its residual by this (block CG) or by half of
+   * this (CG on each right-hand side: the refinement's last step then seldom ends
+   * just above r_tol) */
+  double inner_tol;
   int32_t max_outer; /* refinement steps, at most */
   int32_t max_inner; /* iterations of one inner solve, at most */
   /* inner solver: LFX_MRHS_PER_RHS_CG, CG on every right-hand side with its

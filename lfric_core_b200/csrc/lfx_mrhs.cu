@@ -1284,7 +1284,7 @@ __global__ void __launch_bounds__(256) bcg_small(int mode, BcgSmall* st, double 
 
 struct lfx_mrhs {
   lfx_ctx* ctx = nullptr;
-  int32_t kind = LFX_MRHS_TF32, nrhs = 64, nl = 0, ncell_2d = 0;
+  int32_t nrhs = 64, nl = 0, ncell_2d = 0;
   int64_t undf = 0;
   int32_t npatch = 0, own_max = 0, max_colours = 0;
   int64_t nent = 0;
@@ -1426,7 +1426,8 @@ int lfx_mrhs_create(const lfx_op* op, int32_t kind, int32_t nrhs, int32_t cells_
     for (int c = 0; c < nc; ++c)
       for (int v = 0; v < 4; ++v) vcells[fill[cv[(size_t)c * 4 + v]]++] = c;
   }
-  // compact patches: breadth-first over cells sharing a vertex
+  // compact patches: breadth-first over cells sharing a vertex (their colours, which
+  // the gather does without, are what lfx_mrhs_info reports)
   std::vector<int32_t> patch(nc, -1);
   int npatch = 0;
   {
@@ -1512,7 +1513,6 @@ int lfx_mrhs_create(const lfx_op* op, int32_t kind, int32_t nrhs, int32_t cells_
 
   auto* m = new lfx_mrhs();
   m->ctx = ctx;
-  m->kind = kind;
   m->nrhs = nrhs;
   m->nl = nl;
   m->ncell_2d = nc;
@@ -1970,13 +1970,17 @@ int lfx_mrhs_solve(lfx_mrhs* m, lfx_op* op64, const lfx_vec* diag, const double*
   std::vector<double> r0(nr), rn(nr);
   std::vector<int> act(64, 0), outer_n(nr, 0);
   // With products accurate to FP32 an inner solve meets its tolerance on the
-  // true residual as well, so the steps would end just under r_tol where r_tol
-  // is near a power of inner_tol (products rounded to TF32 fell short and took
-  // a step more): each step goes to half the tolerance, which keeps that
-  // margin (C48 x 30, r_tol 1e-10, inner_tol 1e-2: relative error of the
-  // solution 2.9e-9 without it, 8.0e-11 with it, 8.8e-11 with the rounded
-  // products). Block CG, whose step ends with its slowest right-hand side, has
-  // that margin by itself.
+  // true residual as well, so that the last step of the refinement can end just
+  // under r_tol (products rounded to TF32 fell short and took a step more). CG on
+  // each right-hand side therefore goes to half the tolerance. Largest error of the
+  // solution against FP64, N(0, 1) right-hand sides, inner_tol 1e-2, r_tol 1e-6, 1e-7,
+  // .. 1e-11; whole tolerance / half / rounded products: C24 x 20 2.4e-5 1.6e-7 1.6e-7
+  // 2.4e-9 2.4e-9 1.6e-11 / 3.0e-6 1.3e-6 1.1e-8 1.1e-8 9.3e-11 9.3e-11 / 2.0e-5 2.1e-7
+  // 1.5e-7 2.9e-9 1.6e-9 2.2e-11; C48 x 30 5.5e-5 4.8e-7 4.8e-7 6.2e-9 6.2e-9 4.3e-11 /
+  // 6.5e-6 2.7e-8 2.7e-8 2.7e-8 1.9e-10 1.9e-10 / 1.6e-6 1.6e-6 2.4e-8 2.4e-8 3.0e-10
+  // 3.0e-10, in 3 to 6 steps, 3 to 5 and 4 to 7. Block CG, whose step ends with its
+  // slowest right-hand side, keeps the whole tolerance: half of it gave C48 x 30 at
+  // 1e-8 2.8e-7 for 1.1e-7, 410 iterations for 361.
   const double inner_tol = (block ? 1.0 : 0.5) * cfg->inner_tol;
   rc = outer_residual(m, op64, b, x, ld);
   if (rc) return rc;

@@ -576,7 +576,8 @@ class MultiRhsOperator(_Handle):
         """FP64 refinement around the FP32 CG for all right-hand
         sides (method: MRHS_PER_RHS_CG, or MRHS_BLOCK_CG for 64 right-hand
         sides); b, x: device FP64 arrays, right-hand side r at offset r * ld.
-        Returns one SolveInfo per right-hand side."""
+        An inner solve reduces its residual by inner_tol (block CG) or half of
+        it (CG on each). Returns one SolveInfo per right-hand side."""
         cfg = MrhsCfg(r_tol, inner_tol, max_outer, max_inner, method)
         info = (SolveInfo * self.nrhs)()
         self.ctx.check(self.ctx.L.lfx_mrhs_solve(self.h, op64.h, diag.h, b_ptr, x_ptr, ld,
