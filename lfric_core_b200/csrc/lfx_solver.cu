@@ -836,9 +836,6 @@ int cg_run(lfx_solver* s, T* x, const T* b) {
 // each) and captures them for every new pair of vectors. With eight the C37 x 23
 // W2 solve (12 iterations) took 1167 us, its first pass 1853.
 constexpr int kBicgIters = 4;
-// looks at the state after one graph each, then after two: a longer solve would
-// pay for twice as many
-constexpr int kBicgLooks = 4;
 template <class T>
 int bicgstab_run(lfx_solver* s, T* x, const T* b) {
   lfx_ctx* ctx = s->ctx;
@@ -974,12 +971,10 @@ int bicgstab_run(lfx_solver* s, T* x, const T* b) {
   };
   // no host round trip before the first graph: its kernels idle if the
   // initial residual already ended the solve (device flags)
-  for (int k = 0;; ++k) {
-    // (a timed replay's events are read before the next one records them)
-    if (k >= kBicgLooks && !ctx->time_applies && (rc = run_graph(s, x, b, batch, false))) return rc;
+  do {
     if ((rc = run_graph(s, x, b, batch))) return rc;
-    if (s->h_state->done) return LFX_OK;
-  }
+  } while (!s->h_state->done);
+  return LFX_OK;
 }
 
 // ------------------------------------------------------------------ GMRES
