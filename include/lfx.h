@@ -494,8 +494,8 @@ enum { LFX_MRHS_PER_RHS_CG = 0, LFX_MRHS_BLOCK_CG = 1 };
 typedef struct {
   double r_tol;      /* per right-hand side: ||b - A x|| <= r_tol ||b - A x0|| */
   /* each inner FP32 solve reduces its residual by this (block CG) or by half of
-   * this (CG on each right-hand side: the refinement's last step then seldom ends
-   * just above r_tol) */
+   * this (CG on each right-hand side, so that its last step ends further below
+   * r_tol) */
   double inner_tol;
   int32_t max_outer; /* refinement steps, at most */
   int32_t max_inner; /* iterations of one inner solve, at most */

@@ -833,8 +833,13 @@ int cg_run(lfx_solver* s, T* x, const T* b) {
 
 // ------------------------------------------------------------------ BiCGStab
 // iterations of one graph: a solve ends with up to three idle ones (17 launches
-// each) and captures them for every new pair of vectors. With eight the C37 x 23
-// W2 solve (12 iterations) took 1167 us, its first pass 1853.
+// each, about 20 us an iteration) and captures them for every new pair of vectors;
+// the host's look after a graph costs about 12 us. With eight the C37 x 23 W2 solve
+// (12 iterations) took 1167 us, its first pass 1853. By iterations, with eight and
+// four (C24 x 20 W2, column preconditioner): 1 221, 138 us; 5 373, 363; 12 772, 706; 13
+// 814, 816; 16 926, 932; 20 1214, 1158; 60 3407, 3433; 61 3453, 3550. Two graphs
+// between looks after the sixteenth iteration cost solves of 17 to 28 iterations 2 to
+// 7 % and gave those of 60 2 %.
 constexpr int kBicgIters = 4;
 template <class T>
 int bicgstab_run(lfx_solver* s, T* x, const T* b) {
