@@ -37,6 +37,8 @@ def test_result_follows_its_number(tmp_path, look, race):
     if r.returncode:
         pytest.skip("no thread sanitizer")
     r = subprocess.run([str(exe)], capture_output=True, text=True)
+    if "FATAL: ThreadSanitizer" in r.stderr:  # it cannot map its shadow memory here
+        pytest.skip("the thread sanitizer does not start")
     assert r.stdout == "3.5\n"
     assert ("data race" in r.stderr) == race
 
